@@ -186,14 +186,7 @@ __global__ void __launch_bounds__(kThreads) k_gs_colour(Dims D, Coef<T> C, const
     const T* phi[3] = {p0, p1, p2};
     const T b = ld(C.beta, 0), c = ld(C.gamma, 0);
     T* p = (COMP == 0) ? p0 : (COMP == 1 ? p1 : p2);
-    if constexpr (DM == 3 && !W) {
-        p[nb.s] = face_update3<T, VISC, COMP>(phi, C, rhs, nb, dxsqinv, b, c, omega);
-    } else {
-        T Lp = face_L<T, DM, VISC, COMP, 0, T, W>(phi, C, nb, dxsqinv, b, c);
-        T fac = face_diag<T, DM, VISC, COMP, W>(C, nb, dxsqinv, b, c);
-        T cur = p[nb.s];
-        p[nb.s] = cur + omega * (ld(rhs, nb.s) - Lp) / fac;
-    }
+    p[nb.s] = face_update<T, DM, VISC, COMP, 0, W>(phi, C, rhs, nb, dxsqinv, b, c, omega);
 }
 
 // --------------------------------------------------------------- odd levels
@@ -216,8 +209,7 @@ __global__ void __launch_bounds__(kThreads) k_colour_update(Dims D, Coef<T> C, c
     if (W && wall_face(nb, COMP)) return;
     const T b = ld(C.beta, 0), c = ld(C.gamma, 0);
     T fac = face_diag<T, DM, VISC, COMP, W>(C, nb, dxsqinv, b, c);
-    T cur = p[nb.s];
-    p[nb.s] = cur + omega * (ld(rhs, nb.s) - ld(Lp, nb.s)) / fac;
+    p[nb.s] = gs_update(p[nb.s], omega, ld(rhs, nb.s), ld(Lp, nb.s), fac);
 }
 
 // --------------------------------------------------------------- GS red/black pair (3D)
@@ -257,7 +249,7 @@ __global__ void __launch_bounds__(kThreads) k_gs_pair(Dims D, Coef<T> C, const T
             const Nb nb = make_nb(D, i0 + x, j, k);
             const T Lp = face_L3<T, VISC, COMP>(phi, C, nb, dxsqinv, b, c);
             const T fac = face_diag3<T, VISC, COMP>(C, nb, dxsqinv, b, c);
-            const T v = ld(pc, nb.s) + omega * (ld(rhs, nb.s) - Lp) / fac;
+            const T v = gs_update(ld(pc, nb.s), omega, ld(rhs, nb.s), Lp, fac);
             slot[(ty + 1) * W + x + 1] = v;
             if (kk >= 1 && kk <= TZ) out[nb.s] = v;
         }
@@ -276,7 +268,7 @@ __global__ void __launch_bounds__(kThreads) k_gs_pair(Dims D, Coef<T> C, const T
             const Nb nb = make_nb(D, wrapi(i0 + x, D.nx), wrapi(j0 + y, D.ny), k);
             const T Lp = face_L3<T, VISC, COMP>(phi, C, nb, dxsqinv, b, c);
             const T fac = face_diag3<T, VISC, COMP>(C, nb, dxsqinv, b, c);
-            slot[(y + 1) * W + x + 1] = ld(pc, nb.s) + omega * (ld(rhs, nb.s) - Lp) / fac;
+            slot[(y + 1) * W + x + 1] = gs_update(ld(pc, nb.s), omega, ld(rhs, nb.s), Lp, fac);
         }
     }
     __syncthreads();
@@ -292,7 +284,7 @@ __global__ void __launch_bounds__(kThreads) k_gs_pair(Dims D, Coef<T> C, const T
         const T cur = ld(pc, nb.s);
         const T Lp = face_L3_own<T, VISC, COMP>(cur, nbv, phi, C, nb, dxsqinv, b, c);
         const T fac = face_diag3<T, VISC, COMP>(C, nb, dxsqinv, b, c);
-        out[nb.s] = cur + omega * (ld(rhs, nb.s) - Lp) / fac;
+        out[nb.s] = gs_update(cur, omega, ld(rhs, nb.s), Lp, fac);
     }
 }
 
@@ -314,14 +306,14 @@ __global__ void __launch_bounds__(kThreads) k_jacobi(Dims D, Coef<T> C, const T*
     } else {
         T Lp = face_L<T, DM, VISC, 0, 0, T, W>(phi, C, nb, dxsqinv, b, c);
         T fac = face_diag<T, DM, VISC, 0, W>(C, nb, dxsqinv, b, c);
-        o0[t] = ld(p0, t) + omega * (ld(r0, t) - Lp) / fac;
+        o0[t] = gs_update(ld(p0, t), omega, ld(r0, t), Lp, fac);
     }
     if (W && wall_face(nb, 1)) {
         o1[t] = T(0);
     } else {
         T Lp = face_L<T, DM, VISC, 1, 0, T, W>(phi, C, nb, dxsqinv, b, c);
         T fac = face_diag<T, DM, VISC, 1, W>(C, nb, dxsqinv, b, c);
-        o1[t] = ld(p1, t) + omega * (ld(r1, t) - Lp) / fac;
+        o1[t] = gs_update(ld(p1, t), omega, ld(r1, t), Lp, fac);
     }
     if constexpr (DM == 3) {
         if (W && wall_face(nb, 2)) {
@@ -329,7 +321,7 @@ __global__ void __launch_bounds__(kThreads) k_jacobi(Dims D, Coef<T> C, const T*
         } else {
             T Lp = face_L<T, DM, VISC, 2, 0, T, W>(phi, C, nb, dxsqinv, b, c);
             T fac = face_diag<T, DM, VISC, 2, W>(C, nb, dxsqinv, b, c);
-            o2[t] = ld(p2, t) + omega * (ld(r2, t) - Lp) / fac;
+            o2[t] = gs_update(ld(p2, t), omega, ld(r2, t), Lp, fac);
         }
     }
 }
@@ -345,63 +337,6 @@ __device__ __forceinline__ T fine_resid(const Dims& F, const Coef<T>& C, const T
     Nb nb = make_nb(F, i, j, k);
     T v = face_L<T, DM, VISC, D_, LD>(phi, C, nb, dxsqinv, b, c) - ldp<LD>(rhs, nb.s);
     return v * T(-1);
-}
-
-// coarse face of component COMP at coarse index (i, j, k): the fine-level
-// residual restricted with the 6-point (2D) / 12-point (3D) stencil.  The 12
-// (6) fine residuals are evaluated one at a time (keeps registers low) and
-// summed in the reference's order:
-//   3D: 1/8 (r0+r1+r2+r3) + 1/16 (r4+r5+r6+r7) + 1/16 (r8+r9+r10+r11)
-//   2D: 1/4 (r0+r1) + 1/8 (r2+r3+r4+r5)
-// with normal offsets 0, +1, -1 and the transverse offsets of
-// stag_mg_solver.f90:1063-1078, 1133-1171.
-template <class T, int DM, int VISC, int COMP, int LD = 0>
-__device__ __forceinline__ T restrict_face(const Dims& F, const Coef<T>& C, const T* const rhs[3], const T* const phi[3], int i,
-                                           int j, int k, T dxsqinv) {
-    const T b = ld(C.beta, 0), cc = ld(C.gamma, 0);
-    constexpr int NQ = (DM == 2) ? 2 : 4;
-    // transverse offsets (di, dj, dk) per component
-    int qi[4], qj[4], qk[4];
-    if constexpr (DM == 2) {
-        if (COMP == 0) { qi[0] = 0; qj[0] = 0; qi[1] = 0; qj[1] = 1; }
-        else { qi[0] = 0; qj[0] = 0; qi[1] = 1; qj[1] = 0; }
-        qk[0] = qk[1] = 0;
-    } else {
-        if (COMP == 0) { int a_[4] = {0, 0, 0, 0}, b_[4] = {0, 1, 0, 1}, c_[4] = {0, 0, 1, 1};
-            for (int q = 0; q < 4; ++q) { qi[q] = a_[q]; qj[q] = b_[q]; qk[q] = c_[q]; } }
-        else if (COMP == 1) { int a_[4] = {0, 1, 0, 1}, b_[4] = {0, 0, 0, 0}, c_[4] = {0, 0, 1, 1};
-            for (int q = 0; q < 4; ++q) { qi[q] = a_[q]; qj[q] = b_[q]; qk[q] = c_[q]; } }
-        else { int a_[4] = {0, 1, 0, 1}, b_[4] = {0, 0, 1, 1}, c_[4] = {0, 0, 0, 0};
-            for (int q = 0; q < 4; ++q) { qi[q] = a_[q]; qj[q] = b_[q]; qk[q] = c_[q]; } }
-    }
-    T r[3 * NQ];
-    const int I = 2 * i, J = 2 * j, K = (DM == 3) ? 2 * k : k;
-#pragma unroll 1
-    for (int m = 0; m < 3 * NQ; ++m) {
-        const int nrm = (m < NQ) ? 0 : (m < 2 * NQ ? 1 : -1);
-        const int q = m % NQ;
-        int ii = I + qi[q], jj = J + qj[q], kk = K + qk[q];
-        if (COMP == 0) ii += nrm;
-        else if (COMP == 1) jj += nrm;
-        else kk += nrm;
-        r[m] = fine_resid<T, DM, VISC, COMP, LD>(F, C, phi, rhs[COMP], ii, jj, kk, dxsqinv, b, cc);
-    }
-    if constexpr (DM == 2)
-        return T(0.25) * (r[0] + r[1]) + T(0.125) * (r[2] + r[3] + r[4] + r[5]);
-    else
-        return T(0.125) * (r[0] + r[1] + r[2] + r[3]) + T(0.0625) * (r[4] + r[5] + r[6] + r[7]) +
-               T(0.0625) * (r[8] + r[9] + r[10] + r[11]);
-}
-
-template <class T, int DM, int VISC, int LD = 0>
-__device__ __forceinline__ void restrict_comp(int comp, const Dims& F, const Coef<T>& C, const T* const rhs[3],
-                                              const T* const phi[3], T* const out[3], int t, int i, int j, int k, T dxsqinv) {
-    if (comp == 0)
-        out[0][t] = restrict_face<T, DM, VISC, 0, LD>(F, C, rhs, phi, i, j, k, dxsqinv);
-    else if (comp == 1)
-        out[1][t] = restrict_face<T, DM, VISC, 1, LD>(F, C, rhs, phi, i, j, k, dxsqinv);
-    else if constexpr (DM == 3)
-        out[2][t] = restrict_face<T, DM, VISC, 2, LD>(F, C, rhs, phi, i, j, k, dxsqinv);
 }
 
 // r = (L phi - rhs) * -1 on every face of one level (stag_mg_solver.f90:406-415)
@@ -440,55 +375,40 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 5 : 0) k_residual(D
     }
 }
 
-// 6-point (2D) / 12-point (3D) restriction of precomputed fine residuals,
-// same summation order as restrict_face, for the coarse cell (i, j, k) at
-// coarse index t.  W: coarse wall faces are zero (physbc_domainvel on the
-// restricted residual, stag_mg_solver.f90:439-443); every other coarse face
-// reads fine faces inside the box.  LD: load mode of the fine arrays (ldp).
-template <class T, int DM, bool W = false, int LD = 0>
-__device__ __forceinline__ void restrict_cell(const Dims& F, const T* f0, const T* f1, const T* f2, const Dims& Dc, T* c0, T* c1,
-                                              T* c2, int i, int j, int k, int t) {
-    const int I = 2 * i, J = 2 * j, K = 2 * k;
+// 6-point (2D) / 12-point (3D) restriction of precomputed fine residuals of
+// component COMP (f) to the coarse cell (i, j, k), in the reference's order
+// (stag_mg_solver.f90:1063-1078, 1133-1171):
+//   3D: 1/8 (r0+r1+r2+r3) + 1/16 (r4+r5+r6+r7) + 1/16 (r8+r9+r10+r11)
+//   2D: 1/4 (r0+r1) + 1/8 (r2+r3+r4+r5)
+// with normal offsets 0, +1, -1, the first transverse direction fastest.
+// W: a coarse wall face is zero (physbc_domainvel on the restricted
+// residual, stag_mg_solver.f90:439-443); every other coarse face reads fine
+// faces inside the box.  LD: load mode of the fine array (ldp).
+template <class T, int DM, int COMP, bool W = false, int LD = 0>
+__device__ __forceinline__ T restrict_one(const Dims& F, const T* f, const Dims& Dc, int i, int j, int k) {
     if constexpr (W) {
-        // wall faces first; the others fall through to the periodic formula
-        const int x[3] = {i, j, k};
-        bool wf[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) wf[d] = d < DM && ((Dc.wall >> d) & 1) && x[d] == 0;
-        if (wf[0]) c0[t] = T(0);
-        if (wf[1]) c1[t] = T(0);
-        if (DM == 3 && wf[2]) c2[t] = T(0);
-        if (wf[0]) c0 = nullptr;
-        if (wf[1]) c1 = nullptr;
-        if (wf[2]) c2 = nullptr;
+        const int x = COMP == 0 ? i : (COMP == 1 ? j : k);
+        if (((Dc.wall >> COMP) & 1) && x == 0) return T(0);
     }
-    auto R = [&](const T* f, int ii, int jj, int kk) {
-        ii = wrapi(ii, F.nx);
-        jj = wrapi(jj, F.ny);
-        kk = (DM == 3) ? wrapi(kk, F.nz) : kk;
-        return ldp<LD>(f, ii + F.nx * (jj + F.ny * kk));
+    const int X[3] = {2 * i, 2 * j, DM == 3 ? 2 * k : k};
+    const int n[3] = {F.nx, F.ny, F.nz};
+    constexpr int t1 = COMP == 0 ? 1 : 0, t2 = COMP == 2 ? 1 : 2;
+    // the sum over the transverse corners at normal offset o
+    auto R = [&](int o, int a, int b) {
+        int y[3] = {X[0], X[1], X[2]};
+        y[COMP] += o;
+        y[t1] += a;
+        if constexpr (DM == 3) y[t2] += b;
+        // only a normal offset can leave the box (the transverse corners are 2c, 2c + 1)
+        y[COMP] = wrapi(y[COMP], n[COMP]);
+        return ldp<LD>(f, y[0] + F.nx * (y[1] + F.ny * y[2]));
     };
-    if constexpr (DM == 2) {
-        if (!W || c0)
-        c0[t] = T(0.25) * (R(f0, I, J, k) + R(f0, I, J + 1, k)) +
-                T(0.125) * (R(f0, I + 1, J, k) + R(f0, I + 1, J + 1, k) + R(f0, I - 1, J, k) + R(f0, I - 1, J + 1, k));
-        if (!W || c1)
-        c1[t] = T(0.25) * (R(f1, I, J, k) + R(f1, I + 1, J, k)) +
-                T(0.125) * (R(f1, I, J + 1, k) + R(f1, I + 1, J + 1, k) + R(f1, I, J - 1, k) + R(f1, I + 1, J - 1, k));
-    } else {
-        if (!W || c0)
-        c0[t] = T(0.125) * (R(f0, I, J, K) + R(f0, I, J + 1, K) + R(f0, I, J, K + 1) + R(f0, I, J + 1, K + 1)) +
-                T(0.0625) * (R(f0, I + 1, J, K) + R(f0, I + 1, J + 1, K) + R(f0, I + 1, J, K + 1) + R(f0, I + 1, J + 1, K + 1)) +
-                T(0.0625) * (R(f0, I - 1, J, K) + R(f0, I - 1, J + 1, K) + R(f0, I - 1, J, K + 1) + R(f0, I - 1, J + 1, K + 1));
-        if (!W || c1)
-        c1[t] = T(0.125) * (R(f1, I, J, K) + R(f1, I + 1, J, K) + R(f1, I, J, K + 1) + R(f1, I + 1, J, K + 1)) +
-                T(0.0625) * (R(f1, I, J + 1, K) + R(f1, I + 1, J + 1, K) + R(f1, I, J + 1, K + 1) + R(f1, I + 1, J + 1, K + 1)) +
-                T(0.0625) * (R(f1, I, J - 1, K) + R(f1, I + 1, J - 1, K) + R(f1, I, J - 1, K + 1) + R(f1, I + 1, J - 1, K + 1));
-        if (!W || c2)
-        c2[t] = T(0.125) * (R(f2, I, J, K) + R(f2, I + 1, J, K) + R(f2, I, J + 1, K) + R(f2, I + 1, J + 1, K)) +
-                T(0.0625) * (R(f2, I, J, K + 1) + R(f2, I + 1, J, K + 1) + R(f2, I, J + 1, K + 1) + R(f2, I + 1, J + 1, K + 1)) +
-                T(0.0625) * (R(f2, I, J, K - 1) + R(f2, I + 1, J, K - 1) + R(f2, I, J + 1, K - 1) + R(f2, I + 1, J + 1, K - 1));
-    }
+    if constexpr (DM == 2)
+        return T(0.25) * (R(0, 0, 0) + R(0, 1, 0)) + T(0.125) * (R(1, 0, 0) + R(1, 1, 0) + R(-1, 0, 0) + R(-1, 1, 0));
+    else
+        return T(0.125) * (R(0, 0, 0) + R(0, 1, 0) + R(0, 0, 1) + R(0, 1, 1)) +
+               T(0.0625) * (R(1, 0, 0) + R(1, 1, 0) + R(1, 0, 1) + R(1, 1, 1)) +
+               T(0.0625) * (R(-1, 0, 0) + R(-1, 1, 0) + R(-1, 0, 1) + R(-1, 1, 1));
 }
 
 template <class T, int DM, bool W = false>
@@ -499,7 +419,9 @@ __global__ void __launch_bounds__(kThreads) k_restrict(Dims F, const T* __restri
     const Pos q = pos3(Dc.nx, Dc.ny);
     if (!q.ok) return;
     const int t = q.i + Dc.nx * (q.j + Dc.ny * q.k);
-    restrict_cell<T, DM, W, 0>(F, f0, f1, f2, Dc, c0, c1, c2, q.i, q.j, q.k, t);
+    c0[t] = restrict_one<T, DM, 0, W>(F, f0, Dc, q.i, q.j, q.k);
+    c1[t] = restrict_one<T, DM, 1, W>(F, f1, Dc, q.i, q.j, q.k);
+    if constexpr (DM == 3) c2[t] = restrict_one<T, DM, 2, W>(F, f2, Dc, q.i, q.j, q.k);
 }
 
 // Residual and restriction of one 3D periodic level in one pass
@@ -512,9 +434,13 @@ __global__ void __launch_bounds__(kThreads) k_restrict(Dims F, const T* __restri
 // fine residual r = (L phi - rhs) * -1 that their 12-point restrictions read
 // (the fine faces of the tile plus one face layer on the low and high side
 // normal to each component), then forms the coarse faces from shared memory
-// in restrict_cell's order.  The fine residual never goes to global memory,
+// in restrict_one's order.  The fine residual never goes to global memory,
 // and each one is evaluated once per block (the 2 x 2 x 2-to-1 stencil
 // overlaps only across the block boundary).
+template <class T>
+__device__ __forceinline__ T sum4(T a, T b, T c, T d) { return a + b + c + d; }
+template <class T>
+__device__ __forceinline__ T restrict12(T s0, T s1, T s2) { return T(0.125) * s0 + T(0.0625) * s1 + T(0.0625) * s2; }
 constexpr int RCX = 8, RCY = 4, RCZ = 4;
 template <int COMP>
 struct RTile {  // fine residuals of one component held by the block
@@ -564,19 +490,13 @@ __global__ void __launch_bounds__(kThreads) k_resid_restrict3(Dims F, Coef<T> C,
         const int out = (ci0 + i) + Dc.nx * ((cj0 + j) + Dc.ny * (ck0 + k));
         if (comp == 0) {
             auto R = [&](int ii, int jj, int kk) { return rs[ii + X::NX * (jj + X::NY * kk)]; };
-            c0[out] = T(0.125) * (R(I, J, K) + R(I, J + 1, K) + R(I, J, K + 1) + R(I, J + 1, K + 1)) +
-                      T(0.0625) * (R(I + 1, J, K) + R(I + 1, J + 1, K) + R(I + 1, J, K + 1) + R(I + 1, J + 1, K + 1)) +
-                      T(0.0625) * (R(I - 1, J, K) + R(I - 1, J + 1, K) + R(I - 1, J, K + 1) + R(I - 1, J + 1, K + 1));
+            c0[out] = restrict12(sum4(R(I, J, K), R(I, J + 1, K), R(I, J, K + 1), R(I, J + 1, K + 1)), sum4(R(I + 1, J, K), R(I + 1, J + 1, K), R(I + 1, J, K + 1), R(I + 1, J + 1, K + 1)), sum4(R(I - 1, J, K), R(I - 1, J + 1, K), R(I - 1, J, K + 1), R(I - 1, J + 1, K + 1)));
         } else if (comp == 1) {
             auto R = [&](int ii, int jj, int kk) { return rs[X::N + ii + Y::NX * (jj + Y::NY * kk)]; };
-            c1[out] = T(0.125) * (R(I, J, K) + R(I + 1, J, K) + R(I, J, K + 1) + R(I + 1, J, K + 1)) +
-                      T(0.0625) * (R(I, J + 1, K) + R(I + 1, J + 1, K) + R(I, J + 1, K + 1) + R(I + 1, J + 1, K + 1)) +
-                      T(0.0625) * (R(I, J - 1, K) + R(I + 1, J - 1, K) + R(I, J - 1, K + 1) + R(I + 1, J - 1, K + 1));
+            c1[out] = restrict12(sum4(R(I, J, K), R(I + 1, J, K), R(I, J, K + 1), R(I + 1, J, K + 1)), sum4(R(I, J + 1, K), R(I + 1, J + 1, K), R(I, J + 1, K + 1), R(I + 1, J + 1, K + 1)), sum4(R(I, J - 1, K), R(I + 1, J - 1, K), R(I, J - 1, K + 1), R(I + 1, J - 1, K + 1)));
         } else {
             auto R = [&](int ii, int jj, int kk) { return rs[X::N + Y::N + ii + Z::NX * (jj + Z::NY * kk)]; };
-            c2[out] = T(0.125) * (R(I, J, K) + R(I + 1, J, K) + R(I, J + 1, K) + R(I + 1, J + 1, K)) +
-                      T(0.0625) * (R(I, J, K + 1) + R(I + 1, J, K + 1) + R(I, J + 1, K + 1) + R(I + 1, J + 1, K + 1)) +
-                      T(0.0625) * (R(I, J, K - 1) + R(I + 1, J, K - 1) + R(I, J + 1, K - 1) + R(I + 1, J + 1, K - 1));
+            c2[out] = restrict12(sum4(R(I, J, K), R(I + 1, J, K), R(I, J + 1, K), R(I + 1, J + 1, K)), sum4(R(I, J, K + 1), R(I + 1, J, K + 1), R(I, J + 1, K + 1), R(I + 1, J + 1, K + 1)), sum4(R(I, J, K - 1), R(I + 1, J, K - 1), R(I, J + 1, K - 1), R(I + 1, J + 1, K - 1)));
         }
     }
 }
@@ -629,82 +549,35 @@ __device__ __forceinline__ T pcat(const T* a, const Dims& Dc, int i, int j, int 
         return cat<T, LD>(a, Dc, i, j, k);
 }
 
-// add the interpolated coarse correction to the DM fine faces at (i, j, k);
-// W: fine wall faces keep their zero (physbc_domainvel after the
-// prolongation, stag_mg_solver.f90:681-690)
-template <class T, int DM, int LD = 0, bool W = false>
-__device__ __forceinline__ void prolong_cell(const Dims& Dc, const T* q0, const T* q1, const T* q2, T* f0, T* f1, T* f2, int t,
-                                             int i, int j, int k) {
-    if constexpr (W) {
-        // the fine grid's wall bits are the coarse grid's
-        const int x[3] = {i, j, k};
-        if ((Dc.wall & 1) && x[0] == 0) f0 = nullptr;
-        if (((Dc.wall >> 1) & 1) && x[1] == 0) f1 = nullptr;
-        if constexpr (DM == 3)
-            if (((Dc.wall >> 2) & 1) && x[2] == 0) f2 = nullptr;
-    }
-    const int i2 = i >> 1, j2 = j >> 1, k2 = k >> 1;
+// v plus the interpolated coarse correction of the fine face of component
+// COMP at (i, j, k) (stag_prolongation's weights and order).  W: a fine wall
+// face keeps its zero (physbc_domainvel after the prolongation,
+// stag_mg_solver.f90:681-690); the fine grid's wall bits are the coarse
+// grid's.
+template <class T, int DM, int COMP, int LD = 0, bool W = false>
+__device__ __forceinline__ T prolong_one(const Dims& Dc, const T* q, T v, int i, int j, int k) {
+    const int x[3] = {i, j, k};
+    if constexpr (W)
+        if (((Dc.wall >> COMP) & 1) && x[COMP] == 0) return v;
+    constexpr int t1 = COMP == 0 ? 1 : 0, t2 = COMP == 2 ? 1 : 2;
+    const int c[3] = {i >> 1, j >> 1, DM == 3 ? k >> 1 : k};
+    const int o1 = (x[t1] & 1) ? 1 : -1, o2 = (DM == 3 && (x[t2] & 1)) ? 1 : -1;
+    auto Q = [&](int nrm, int a, int b) {
+        int y[3] = {c[0], c[1], c[2]};
+        y[COMP] += nrm;
+        y[t1] += a;
+        if constexpr (DM == 3) y[t2] += b;
+        return pcat<T, LD, W, COMP>(q, Dc, y[0], y[1], y[2]);
+    };
     if constexpr (DM == 2) {
-        if (!W || f0) {
-            int joff = ((j & 1) == 0) ? -1 : 1;
-            T v = (LD == 2) ? __ldcg(f0 + t) : f0[t];
-            if ((i & 1) == 0)
-                v = v + T(0.75) * pcat<T, LD, W, 0>(q0, Dc, i2, j2, k) + T(0.25) * pcat<T, LD, W, 0>(q0, Dc, i2, j2 + joff, k);
-            else
-                v = v + T(0.375) * pcat<T, LD, W, 0>(q0, Dc, i2, j2, k) + T(0.125) * pcat<T, LD, W, 0>(q0, Dc, i2, j2 + joff, k) + T(0.375) * pcat<T, LD, W, 0>(q0, Dc, i2 + 1, j2, k) +
-                    T(0.125) * pcat<T, LD, W, 0>(q0, Dc, i2 + 1, j2 + joff, k);
-            f0[t] = v;
-        }
-        if (!W || f1) {
-            int ioff = ((i & 1) == 0) ? -1 : 1;
-            T v = (LD == 2) ? __ldcg(f1 + t) : f1[t];
-            if ((j & 1) == 0)
-                v = v + T(0.75) * pcat<T, LD, W, 1>(q1, Dc, i2, j2, k) + T(0.25) * pcat<T, LD, W, 1>(q1, Dc, i2 + ioff, j2, k);
-            else
-                v = v + T(0.375) * pcat<T, LD, W, 1>(q1, Dc, i2, j2, k) + T(0.125) * pcat<T, LD, W, 1>(q1, Dc, i2 + ioff, j2, k) + T(0.375) * pcat<T, LD, W, 1>(q1, Dc, i2, j2 + 1, k) +
-                    T(0.125) * pcat<T, LD, W, 1>(q1, Dc, i2 + ioff, j2 + 1, k);
-            f1[t] = v;
-        }
+        if ((x[COMP] & 1) == 0) return v + T(0.75) * Q(0, 0, 0) + T(0.25) * Q(0, o1, 0);
+        return v + T(0.375) * Q(0, 0, 0) + T(0.125) * Q(0, o1, 0) + T(0.375) * Q(1, 0, 0) + T(0.125) * Q(1, o1, 0);
     } else {
         const T n16 = T(9.0 / 16.0), t16 = T(3.0 / 16.0), o16 = T(1.0 / 16.0);
         const T n32 = T(9.0 / 32.0), t32 = T(3.0 / 32.0), o32 = T(1.0 / 32.0);
-        const int ioff = ((i & 1) == 0) ? -1 : 1, joff = ((j & 1) == 0) ? -1 : 1, koff = ((k & 1) == 0) ? -1 : 1;
-        if (!W || f0) {
-            T v = (LD == 2) ? __ldcg(f0 + t) : f0[t];
-            if ((i & 1) == 0)
-                v = v + n16 * pcat<T, LD, W, 0>(q0, Dc, i2, j2, k2) + t16 * pcat<T, LD, W, 0>(q0, Dc, i2, j2 + joff, k2) + t16 * pcat<T, LD, W, 0>(q0, Dc, i2, j2, k2 + koff) +
-                    o16 * pcat<T, LD, W, 0>(q0, Dc, i2, j2 + joff, k2 + koff);
-            else
-                v = v + n32 * pcat<T, LD, W, 0>(q0, Dc, i2, j2, k2) + t32 * pcat<T, LD, W, 0>(q0, Dc, i2, j2 + joff, k2) + t32 * pcat<T, LD, W, 0>(q0, Dc, i2, j2, k2 + koff) +
-                    o32 * pcat<T, LD, W, 0>(q0, Dc, i2, j2 + joff, k2 + koff) + n32 * pcat<T, LD, W, 0>(q0, Dc, i2 + 1, j2, k2) +
-                    t32 * pcat<T, LD, W, 0>(q0, Dc, i2 + 1, j2 + joff, k2) + t32 * pcat<T, LD, W, 0>(q0, Dc, i2 + 1, j2, k2 + koff) +
-                    o32 * pcat<T, LD, W, 0>(q0, Dc, i2 + 1, j2 + joff, k2 + koff);
-            f0[t] = v;
-        }
-        if (!W || f1) {
-            T v = (LD == 2) ? __ldcg(f1 + t) : f1[t];
-            if ((j & 1) == 0)
-                v = v + n16 * pcat<T, LD, W, 1>(q1, Dc, i2, j2, k2) + t16 * pcat<T, LD, W, 1>(q1, Dc, i2 + ioff, j2, k2) + t16 * pcat<T, LD, W, 1>(q1, Dc, i2, j2, k2 + koff) +
-                    o16 * pcat<T, LD, W, 1>(q1, Dc, i2 + ioff, j2, k2 + koff);
-            else
-                v = v + n32 * pcat<T, LD, W, 1>(q1, Dc, i2, j2, k2) + t32 * pcat<T, LD, W, 1>(q1, Dc, i2 + ioff, j2, k2) + t32 * pcat<T, LD, W, 1>(q1, Dc, i2, j2, k2 + koff) +
-                    o32 * pcat<T, LD, W, 1>(q1, Dc, i2 + ioff, j2, k2 + koff) + n32 * pcat<T, LD, W, 1>(q1, Dc, i2, j2 + 1, k2) +
-                    t32 * pcat<T, LD, W, 1>(q1, Dc, i2 + ioff, j2 + 1, k2) + t32 * pcat<T, LD, W, 1>(q1, Dc, i2, j2 + 1, k2 + koff) +
-                    o32 * pcat<T, LD, W, 1>(q1, Dc, i2 + ioff, j2 + 1, k2 + koff);
-            f1[t] = v;
-        }
-        if (!W || f2) {
-            T v = (LD == 2) ? __ldcg(f2 + t) : f2[t];
-            if ((k & 1) == 0)
-                v = v + n16 * pcat<T, LD, W, 2>(q2, Dc, i2, j2, k2) + t16 * pcat<T, LD, W, 2>(q2, Dc, i2 + ioff, j2, k2) + t16 * pcat<T, LD, W, 2>(q2, Dc, i2, j2 + joff, k2) +
-                    o16 * pcat<T, LD, W, 2>(q2, Dc, i2 + ioff, j2 + joff, k2);
-            else
-                v = v + n32 * pcat<T, LD, W, 2>(q2, Dc, i2, j2, k2) + t32 * pcat<T, LD, W, 2>(q2, Dc, i2 + ioff, j2, k2) + t32 * pcat<T, LD, W, 2>(q2, Dc, i2, j2 + joff, k2) +
-                    o32 * pcat<T, LD, W, 2>(q2, Dc, i2 + ioff, j2 + joff, k2) + n32 * pcat<T, LD, W, 2>(q2, Dc, i2, j2, k2 + 1) +
-                    t32 * pcat<T, LD, W, 2>(q2, Dc, i2 + ioff, j2, k2 + 1) + t32 * pcat<T, LD, W, 2>(q2, Dc, i2, j2 + joff, k2 + 1) +
-                    o32 * pcat<T, LD, W, 2>(q2, Dc, i2 + ioff, j2 + joff, k2 + 1);
-            f2[t] = v;
-        }
+        if ((x[COMP] & 1) == 0) return v + n16 * Q(0, 0, 0) + t16 * Q(0, o1, 0) + t16 * Q(0, 0, o2) + o16 * Q(0, o1, o2);
+        return v + n32 * Q(0, 0, 0) + t32 * Q(0, o1, 0) + t32 * Q(0, 0, o2) + o32 * Q(0, o1, o2) + n32 * Q(1, 0, 0) +
+               t32 * Q(1, o1, 0) + t32 * Q(1, 0, o2) + o32 * Q(1, o1, o2);
     }
 }
 
@@ -716,7 +589,9 @@ __global__ void __launch_bounds__(kThreads) k_prolong_add(Dims F, Dims Dc, const
     const Pos q = pos3(F.nx, F.ny);
     if (!q.ok) return;
     const int t = q.i + F.nx * (q.j + F.ny * q.k);
-    prolong_cell<T, DM, 0, W>(Dc, q0, q1, q2, f0, f1, f2, t, q.i, q.j, q.k);
+    f0[t] = prolong_one<T, DM, 0, 0, W>(Dc, q0, f0[t], q.i, q.j, q.k);
+    f1[t] = prolong_one<T, DM, 1, 0, W>(Dc, q1, f1[t], q.i, q.j, q.k);
+    if constexpr (DM == 3) f2[t] = prolong_one<T, DM, 2, 0, W>(Dc, q2, f2[t], q.i, q.j, q.k);
 }
 
 // --------------------------------------------------------------- coefficient coarsening
@@ -799,22 +674,54 @@ __global__ void __launch_bounds__(kThreads) k_coarsen_edges_w(Dims F, Dims Dc, c
 }
 
 // --------------------------------------------------------------- pressure multigrid
-template <class T, int DM, int LD = 0>
-__device__ __forceinline__ T cc_lap(const T* const a[3], const T* phi, const Nb& n, T dxsqinv) {
-    const int s = n.s;
-    const T p = ldp<LD>(phi, s);
-    T v = (ld(a[0], s + n.op[0]) * (ldp<LD>(phi, s + n.op[0]) - p) - ld(a[0], s) * (p - ldp<LD>(phi, s + n.om[0]))) +
-          (ld(a[1], s + n.op[1]) * (ldp<LD>(phi, s + n.op[1]) - p) - ld(a[1], s) * (p - ldp<LD>(phi, s + n.om[1])));
-    if constexpr (DM == 3)
-        v = v + (ld(a[2], s + n.op[2]) * (ldp<LD>(phi, s + n.op[2]) - p) - ld(a[2], s) * (p - ldp<LD>(phi, s + n.om[2])));
+// div(a grad phi) of a cell from its values: a = the face coefficients
+// {-x, +x, -y, +y, -z, +z}, nb = the neighbours {+x, -x, ...}
+template <class T, int DM>
+__device__ __forceinline__ T cc_lap_vals(const T (&a)[6], T p, const T (&nb)[6], T dxsqinv) {
+    T v = (a[1] * (nb[0] - p) - a[0] * (p - nb[1])) + (a[3] * (nb[2] - p) - a[2] * (p - nb[3]));
+    if constexpr (DM == 3) v = v + (a[5] * (nb[4] - p) - a[4] * (p - nb[5]));
     return v * dxsqinv;
 }
 template <class T, int DM>
-__device__ __forceinline__ T cc_diag(const T* const a[3], const Nb& n, T dxsqinv) {
-    const int s = n.s;
-    T sum = ld(a[0], s) + ld(a[0], s + n.op[0]) + ld(a[1], s) + ld(a[1], s + n.op[1]);
-    if constexpr (DM == 3) sum = sum + ld(a[2], s) + ld(a[2], s + n.op[2]);
+__device__ __forceinline__ T cc_diag_vals(const T (&a)[6], T dxsqinv) {
+    T sum = a[0] + a[1] + a[2] + a[3];
+    if constexpr (DM == 3) sum = sum + a[4] + a[5];
     return -(sum * dxsqinv);
+}
+template <class T, int DM, int LD = 0>
+__device__ __forceinline__ void cc_nb(const T* phi, const Nb& n, T (&nb)[6]) {
+#pragma unroll
+    for (int d = 0; d < DM; ++d) {
+        nb[2 * d] = ldp<LD>(phi, n.s + n.op[d]);
+        nb[2 * d + 1] = ldp<LD>(phi, n.s + n.om[d]);
+    }
+}
+// U: every face coefficient is c (the value each load would return)
+template <class T, int DM, bool U>
+__device__ __forceinline__ void cc_coef(const T* const a[3], T c, const Nb& n, T (&k)[6]) {
+#pragma unroll
+    for (int d = 0; d < DM; ++d) {
+        k[2 * d] = U ? c : ld(a[d], n.s);
+        k[2 * d + 1] = U ? c : ld(a[d], n.s + n.op[d]);
+    }
+}
+// rhs - div(a grad phi) at a cell
+template <class T, int DM, bool U = false, int LD = 0>
+__device__ __forceinline__ T cc_resid(const T* const a[3], T c, const T* phi, const T* rhs, const Nb& n, T dxsqinv) {
+    T k[6], nb[6];
+    cc_coef<T, DM, U>(a, c, n, k);
+    cc_nb<T, DM, LD>(phi, n, nb);
+    return ldp<LD>(rhs, n.s) - cc_lap_vals<T, DM>(k, ldp<LD>(phi, n.s), nb, dxsqinv);
+}
+// one Gauss-Seidel update of a cell
+template <class T, int DM, bool U = false, int LD = 0>
+__device__ __forceinline__ T cc_update(const T* const a[3], T c, const T* phi, const T* rhs, const Nb& n, T dxsqinv) {
+    T k[6], nb[6];
+    cc_coef<T, DM, U>(a, c, n, k);
+    cc_nb<T, DM, LD>(phi, n, nb);
+    const T p = ldp<LD>(phi, n.s);
+    const T res = ldp<LD>(rhs, n.s) - cc_lap_vals<T, DM>(k, p, nb, dxsqinv);
+    return p + res / cc_diag_vals<T, DM>(k, dxsqinv);
 }
 
 // flag = 1 when an entry of a0, a1 or a2 (a1, a2 may be null) differs from
@@ -835,24 +742,6 @@ __global__ void k_uniform_check(const T* __restrict__ a0, const T* __restrict__ 
     if (diff) atomicOr(flag, 1);
 }
 
-// the same two expressions with every face coefficient equal to c (the
-// value each load would return: the same operations, the same bits)
-template <class T, int DM, int LD = 0>
-__device__ __forceinline__ T cc_lap_u(T c, const T* phi, const Nb& n, T dxsqinv) {
-    const int s = n.s;
-    const T p = ldp<LD>(phi, s);
-    T v = (c * (ldp<LD>(phi, s + n.op[0]) - p) - c * (p - ldp<LD>(phi, s + n.om[0]))) +
-          (c * (ldp<LD>(phi, s + n.op[1]) - p) - c * (p - ldp<LD>(phi, s + n.om[1])));
-    if constexpr (DM == 3) v = v + (c * (ldp<LD>(phi, s + n.op[2]) - p) - c * (p - ldp<LD>(phi, s + n.om[2])));
-    return v * dxsqinv;
-}
-template <class T, int DM>
-__device__ __forceinline__ T cc_diag_u(T c, T dxsqinv) {
-    T sum = c + c + c + c;
-    if constexpr (DM == 3) sum = sum + c + c;
-    return -(sum * dxsqinv);
-}
-
 // U: every face coefficient equals cu (the arrays a0..a2 are not read);
 // reverse: the blocks take the planes in decreasing order (see k_gs_colour)
 template <class T, int DM, bool U = false>
@@ -864,16 +753,8 @@ __global__ void __launch_bounds__(kThreads) k_cc_smooth(Dims D, const T* a0, con
     const int j = q.j, k = reverse ? (int)gridDim.z - 1 - q.k : q.k;
     const int i = 2 * q.i + ((j + ck<DM>(k) + parity) & 1);
     Nb nb = make_nb(D, i, j, k);
-    if constexpr (U) {
-        T res = ld(rhs, nb.s) - cc_lap_u<T, DM>(cu, phi, nb, dxsqinv);
-        T cur = phi[nb.s];
-        phi[nb.s] = cur + res / cc_diag_u<T, DM>(cu, dxsqinv);
-    } else {
-        const T* a[3] = {a0, a1, a2};
-        T res = ld(rhs, nb.s) - cc_lap<T, DM>(a, phi, nb, dxsqinv);
-        T cur = phi[nb.s];
-        phi[nb.s] = cur + res / cc_diag<T, DM>(a, nb, dxsqinv);
-    }
+    const T* a[3] = {a0, a1, a2};
+    phi[nb.s] = cc_update<T, DM, U>(a, cu, phi, rhs, nb, dxsqinv);
 }
 
 // one colour of the pressure smoother on an odd level: new values from the
@@ -886,9 +767,7 @@ __global__ void __launch_bounds__(kThreads) k_cc_smooth_odd(Dims D, const T* a0,
     if (!q.ok || ((q.i + q.j + ck<DM>(q.k)) & 1) != parity) return;
     Nb nb = make_nb(D, q.i, q.j, q.k);
     const T* a[3] = {a0, a1, a2};
-    T res = ld(rhs, nb.s) - cc_lap<T, DM>(a, phi, nb, dxsqinv);
-    T cur = phi[nb.s];
-    out[nb.s] = cur + res / cc_diag<T, DM>(a, nb, dxsqinv);
+    out[nb.s] = cc_update<T, DM>(a, T(0), phi, rhs, nb, dxsqinv);
 }
 
 template <class T>
@@ -898,13 +777,6 @@ __global__ void __launch_bounds__(kThreads) k_copy_parity(Dims D, const T* __res
     if (!q.ok || ((q.i + q.j + (D.dm == 3 ? q.k : 0)) & 1) != parity) return;
     const int s = q.i + D.nx * (q.j + D.ny * q.k);
     out[s] = in[s];
-}
-
-template <class T, int DM, int LD = 0>
-__device__ __forceinline__ T cc_res_at(const Dims& F, const T* const a[3], const T* phi, const T* rhs, int i, int j, int k,
-                                       T dxsqinv) {
-    Nb nb = make_nb(F, i, j, k);
-    return ldp<LD>(rhs, nb.s) - cc_lap<T, DM, LD>(a, phi, nb, dxsqinv);
 }
 
 template <class T, int DM, bool U = false>
@@ -919,12 +791,7 @@ __global__ void __launch_bounds__(kThreads) k_cc_residual_restrict(Dims F, const
     const T* a[3] = {a0, a1, a2};
     const int I = 2 * i, J = 2 * j, K = 2 * k;
     auto res_at = [&](int ii, int jj, int kk) -> T {
-        if constexpr (U) {
-            Nb nb = make_nb(F, ii, jj, kk);
-            return ld(rhs, nb.s) - cc_lap_u<T, DM>(cu, phi, nb, dxsqinv);
-        } else {
-            return cc_res_at<T, DM>(F, a, phi, rhs, ii, jj, kk, dxsqinv);
-        }
+        return cc_resid<T, DM, U>(a, cu, phi, rhs, make_nb(F, ii, jj, kk), dxsqinv);
     };
 #define R(ii, jj, kk) res_at(ii, jj, kk)
     if constexpr (DM == 2)
@@ -952,7 +819,10 @@ __global__ void __launch_bounds__(kThreads) k_neg_cc_lap(Dims D, const T* a0, co
     if (!q.ok) return;
     Nb nb = make_nb(D, q.i, q.j, q.k);
     const T* a[3] = {a0, a1, a2};
-    out[nb.s] = -cc_lap<T, DM>(a, phi, nb, dxsqinv);
+    T k[6], nbv[6];
+    cc_coef<T, DM, false>(a, T(0), nb, k);
+    cc_nb<T, DM>(phi, nb, nbv);
+    out[nb.s] = -cc_lap_vals<T, DM>(k, ld(phi, nb.s), nbv, dxsqinv);
 }
 
 // --------------------------------------------------------------- div / grad pieces

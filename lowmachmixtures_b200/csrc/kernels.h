@@ -114,14 +114,15 @@ template <class T>
 void wl_prolong_add(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const phi_c[3], T* const phi_f[3], cudaStream_t s);
 
 // The coarse end of a V-cycle (levels L[0..nl-1], L[0] already holding its
-// rhs) in one single-block launch with every level in shared memory (tail.cuh).
+// rhs) in one single-block launch with every level in shared memory
+// (tail.cuh).  zero: L[0]'s phi is zero (its array is written, not read).
 template <class T>
 cudaError_t launch_vcycle_tail(const LevelDev<T>* L, int nl, int visc, int nu1, int nu2, int nub, int smoother, double omega,
-                               cudaStream_t s);
+                               cudaStream_t s, bool zero);
 template <class T>
-cudaError_t launch_ccmg_tail(const LevelDev<T>* L, int nl, int nu1, int nu2, int nub, cudaStream_t s);
+cudaError_t launch_ccmg_tail(const LevelDev<T>* L, int nl, int nu1, int nu2, int nub, cudaStream_t s, bool zero);
 template <class T>
-size_t tail_smem_bytes(const LevelDev<T>* L, int nl, bool stag, bool jacobi);
+size_t tail_smem_bytes(const LevelDev<T>* L, int nl, bool stag);
 
 // ---- pressure multigrid (this library's cell-centred V-cycle) ----
 // reverse: the launch takes the planes in decreasing order (same values)

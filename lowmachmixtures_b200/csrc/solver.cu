@@ -861,11 +861,10 @@ int tail_start(lmm_handle* h, const std::vector<LevelDev<T>>& L, int nl, bool st
     const int cells = h->knobs.tail_cells == 0 ? (stag ? vel_cells : 4096) : h->knobs.tail_cells;
     if (cells < 0) return nl;
     const size_t budget = (size_t)(h->knobs.tail_smem_kb > 0 ? h->knobs.tail_smem_kb : 200) * 1024;
-    const bool jacobi = stag && h->knobs.stag_mg_smoother == 0;
     const int64_t inst = (h->dm == 2) ? h->batch : 1;  // a 2D batch: one tail block per instance
     int lc = nl;
     while (lc > 0 && nl - (lc - 1) <= 12 && L[lc - 1].n / inst <= cells &&
-           tail_smem_bytes<T>(&L[lc - 1], nl - (lc - 1), stag, jacobi) <= budget)
+           tail_smem_bytes<T>(&L[lc - 1], nl - (lc - 1), stag) <= budget)
         --lc;
     return lc;
 }
@@ -876,8 +875,8 @@ void vcycle(lmm_handle* h, std::vector<LevelDev<T>>& L) {
     const lmm_knobs& K = h->knobs;
     const int nl = h->nlev;
     const int lc = tail_start<T>(h, L, nl, true);
-    // coarse-level initial guesses are zero; the tail zeroes the levels below its first
-    for (int l = 1; l <= std::min(lc, nl - 1); ++l)
+    // coarse-level initial guesses are zero; the tail takes those of its own levels as zero
+    for (int l = 1; l < std::min(lc, nl); ++l)
         for (int d = 0; d < h->dm; ++d) LMM_CK(cudaMemsetAsync(L[l].phi[d], 0, L[l].n * sizeof(T), h->stream));
     for (int l = 0; l < lc && l < nl - 1; ++l) {
         smooth<T>(h, L[l], K.stag_mg_nsmooths_down);
@@ -887,7 +886,7 @@ void vcycle(lmm_handle* h, std::vector<LevelDev<T>>& L) {
     }
     if (lc < nl) {
         LMM_CK(launch_vcycle_tail<T>(&L[lc], nl - lc, K.visc_type, K.stag_mg_nsmooths_down, K.stag_mg_nsmooths_up,
-                                     K.stag_mg_nsmooths_bottom, K.stag_mg_smoother, K.stag_mg_omega, h->stream));
+                                     K.stag_mg_nsmooths_bottom, K.stag_mg_smoother, K.stag_mg_omega, h->stream, lc > 0));
         check_launch();
     } else {
         smooth<T>(h, L[nl - 1], K.stag_mg_nsmooths_bottom);
@@ -984,7 +983,7 @@ void macproject(lmm_handle* h) {
     const int lc = tail_start<T>(h, L, nl, false);
     LMM_CK(cudaMemsetAsync(L[0].pphi, 0, L[0].n * sizeof(T), h->stream));
     for (int vc = 0; vc < K.mg_max_vcycles; ++vc) {
-        for (int l = 1; l <= std::min(lc, nl - 1); ++l) LMM_CK(cudaMemsetAsync(L[l].pphi, 0, L[l].n * sizeof(T), h->stream));
+        for (int l = 1; l < std::min(lc, nl); ++l) LMM_CK(cudaMemsetAsync(L[l].pphi, 0, L[l].n * sizeof(T), h->stream));
         for (int l = 0; l < lc && l < nl - 1; ++l) {
             cc_smooth<T>(h, L[l], K.mg_nsmooths_down);
             launch_cc_residual_restrict<T>(L[l], L[l + 1], h->stream);
@@ -992,7 +991,7 @@ void macproject(lmm_handle* h) {
         }
         if (lc < nl) {
             LMM_CK(launch_ccmg_tail<T>(&L[lc], nl - lc, K.mg_nsmooths_down, K.mg_nsmooths_up, K.mg_nsmooths_bottom,
-                                       h->stream));
+                                       h->stream, lc > 0 || vc == 0));
             check_launch();
         } else {
             cc_smooth<T>(h, L[nl - 1], K.mg_nsmooths_bottom);

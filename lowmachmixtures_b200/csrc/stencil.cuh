@@ -294,156 +294,25 @@ template <> struct Perm3<0> { static constexpr int t1 = 1, t2 = 2, e1 = 0, e2 = 
 template <> struct Perm3<1> { static constexpr int t1 = 0, t2 = 2, e1 = 0, e2 = 2; };
 template <> struct Perm3<2> { static constexpr int t1 = 0, t2 = 1, e1 = 1, e2 = 2; };
 
+// ------------------------------------------------------------ rounding of the face arithmetic
+// Every kernel that evaluates a face (colour launches, residuals, the
+// single-block tails, the fused pairs) goes through the value functions
+// below, so a face has the same bits in whichever kernel evaluates it.  FP64:
+// the Fortran's operand order, one rounding per operation (the units are
+// built without contraction).  FP32: the same expressions with the compiler's
+// contractions, which are those of the expression and not of the kernel
+// around it (the mixed solves compare bit for bit across kernels).
+
 // ------------------------------------------------------------------ 3D
-// The face value with the own component's centre p0 and its six neighbours
-// nb = {+x, -x, +y, -y, +z, -z} supplied by the caller (global memory for the
-// plain kernels, shared memory for the fused red/black pair); the other two
-// components and the coefficients are read through phi / C.
-template <class T, int VISC, int D, int LD = 0, class TP = T, bool W = false>
-__device__ __forceinline__ T face_L3_own(const T p0, const T (&nb)[6], const TP* const phi[3], const Coef<T>& C, const Nb& n,
-                                         T dxsqinv, T b, T c) {
-    constexpr int t1 = Perm3<D>::t1, t2 = Perm3<D>::t2, e1 = Perm3<D>::e1, e2 = Perm3<D>::e2;
-    const T onethird = T(1) / T(3), twothirds = T(2) / T(3), fourthirds = T(4) / T(3);
-    const int s = n.s;
-    const T a = alpha_at(C, D, s);
-    if (VISC == 1) {
-        T nbs = nb[0] + nb[1] + nb[2] + nb[3] + nb[4] + nb[5];
-        return p0 * (a + T(6) * b * dxsqinv) - nbs * b * dxsqinv;
-    }
-    const TP* q1 = phi[t1];
-    const TP* q2 = phi[t2];
-    const T ppd = nb[2 * D], pmd = nb[2 * D + 1];
-    const T pp1 = nb[2 * t1], pm1 = nb[2 * t1 + 1];
-    const T pp2 = nb[2 * t2], pm2 = nb[2 * t2 + 1];
-    // cross terms q(i,+t) , q(i) , q(i-d,+t) , q(i-d)
-    T c10 = (T)ldp<LD>(q1, s + n.op[t1]), c11 = (T)ldp<LD>(q1, s), c12 = (T)ldp<LD>(q1, s + n.om[D] + n.op[t1]), c13 = (T)ldp<LD>(q1, s + n.om[D]);
-    T c20 = (T)ldp<LD>(q2, s + n.op[t2]), c21 = (T)ldp<LD>(q2, s), c22 = (T)ldp<LD>(q2, s + n.om[D] + n.op[t2]), c23 = (T)ldp<LD>(q2, s + n.om[D]);
-    if constexpr (W) {
-        // component t across its own wall at +t is zero (the face is not a wall face, so -d stays inside)
-        const int m1 = wall_mul(n, t1, t1, true), m2 = wall_mul(n, t2, t2, true);
-        c10 = wapply(m1, c10);
-        c12 = wapply(m1, c12);
-        c20 = wapply(m2, c20);
-        c22 = wapply(m2, c22);
-    }
-    if (VISC == 2) {
-        return p0 * (a + T(8) * b * dxsqinv) -
-               (T(2) * ppd + T(2) * pmd + pp1 + pm1 + pp2 + pm2 + c10 - c11 - c12 + c13 + c20 - c21 - c22 + c23) * b * dxsqinv;
-    }
-    if (VISC == 3) {
-        T nbt;
-        if (D == 0) nbt = pp1 + pm1 + pp2 + pm2;              // j+1, j-1, k+1, k-1
-        else if (D == 1) nbt = pp1 + pm1 + pp2 + pm2;         // i+1, i-1, k+1, k-1
-        else nbt = pp1 + pm1 + pp2 + pm2;                     // i+1, i-1, j+1, j-1
-        return p0 * (a + (T(20) * b * onethird + T(2) * c) * dxsqinv) -
-               ((ppd + pmd) * (fourthirds * b + c) + nbt * b +
-                (c10 - c11 - c12 + c13 + c20 - c21 - c22 + c23) * (onethird * b + c)) * dxsqinv;
-    }
-    const T be = ld(C.beta, s), bm = ld(C.beta, s + n.om[D]);
-    const T E1 = ld(C.bed[e1], W ? edge_at(n, e1, -1) : s), E1p = ld(C.bed[e1], W ? edge_at(n, e1, t1) : s + n.op[t1]);
-    const T E2 = ld(C.bed[e2], W ? edge_at(n, e2, -1) : s), E2p = ld(C.bed[e2], W ? edge_at(n, e2, t2) : s + n.op[t2]);
-    if (VISC == -1) {
-        return p0 * (a + (be + bm + E1 + E1p + E2 + E2p) * dxsqinv) -
-               (ppd * be + pmd * bm + pp1 * E1p + pm1 * E1 + pp2 * E2p + pm2 * E2) * dxsqinv;
-    }
-    if (VISC == -2) {
-        return p0 * (a + (T(2) * be + T(2) * bm + E1 + E1p + E2 + E2p) * dxsqinv) -
-               (T(2) * ppd * be + T(2) * pmd * bm + pp1 * E1p + pm1 * E1 + pp2 * E2p + pm2 * E2 + c10 * E1p - c11 * E1 - c12 * E1p +
-                c13 * E1 + c20 * E2p - c21 * E2 - c22 * E2p + c23 * E2) * dxsqinv;
-    }
-    // VISC == -3
-    const T g = ld(C.gamma, s), gm = ld(C.gamma, s + n.om[D]);
-    return p0 * (a + (fourthirds * be + g + fourthirds * bm + gm + E1 + E1p + E2 + E2p) * dxsqinv) -
-           (ppd * (fourthirds * be + g) + pmd * (fourthirds * bm + gm) + pp1 * E1p + pm1 * E1 + pp2 * E2p + pm2 * E2 +
-            c10 * (E1p - twothirds * be + g) - c11 * (E1 - twothirds * be + g) - c12 * (E1p - twothirds * bm + gm) +
-            c13 * (E1 - twothirds * bm + gm) + c20 * (E2p - twothirds * be + g) - c21 * (E2 - twothirds * be + g) -
-            c22 * (E2p - twothirds * bm + gm) + c23 * (E2 - twothirds * bm + gm)) * dxsqinv;
-}
-
-template <class T, int VISC, int D, int LD = 0, class TP = T, bool W = false>
-__device__ __forceinline__ T face_L3(const TP* const phi[3], const Coef<T>& C, const Nb& n, T dxsqinv, T b, T c) {
-    const TP* p = phi[D];
-    const int s = n.s;
-    const T p0 = (T)ldp<LD>(p, s);
-    T nb[6] = {(T)ldp<LD>(p, s + n.op[0]), (T)ldp<LD>(p, s + n.om[0]), (T)ldp<LD>(p, s + n.op[1]),
-               (T)ldp<LD>(p, s + n.om[1]), (T)ldp<LD>(p, s + n.op[2]), (T)ldp<LD>(p, s + n.om[2])};
-    if constexpr (W) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            nb[2 * d] = wapply(wall_mul(n, D, d, true), nb[2 * d]);
-            nb[2 * d + 1] = wapply(wall_mul(n, D, d, false), nb[2 * d + 1]);
-        }
-    }
-    return face_L3_own<T, VISC, D, LD, TP, W>(p0, nb, phi, C, n, dxsqinv, b, c);
-}
-
-template <class T, int VISC, int D, bool W = false>
-__device__ __forceinline__ T face_diag3(const Coef<T>& C, const Nb& n, T dxsqinv, T b, T c) {
-    constexpr int t1 = Perm3<D>::t1, t2 = Perm3<D>::t2, e1 = Perm3<D>::e1, e2 = Perm3<D>::e2;
-    const int s = n.s;
-    const T a = alpha_at(C, D, s);
-    if (VISC == 1) return a + T(6) * b * dxsqinv;
-    if (VISC == 2) return a + T(8) * b * dxsqinv;
-    if (VISC == 3) return a + (T(20) / T(3) * b + T(2) * c) * dxsqinv;
-    const T be = ld(C.beta, s), bm = ld(C.beta, s + n.om[D]);
-    const T E1 = ld(C.bed[e1], W ? edge_at(n, e1, -1) : s), E1p = ld(C.bed[e1], W ? edge_at(n, e1, t1) : s + n.op[t1]);
-    const T E2 = ld(C.bed[e2], W ? edge_at(n, e2, -1) : s), E2p = ld(C.bed[e2], W ? edge_at(n, e2, t2) : s + n.op[t2]);
-    if (VISC == -1) return a + (be + bm + E1 + E1p + E2 + E2p) * dxsqinv;
-    if (VISC == -2) return a + (T(2) * be + T(2) * bm + E1 + E1p + E2 + E2p) * dxsqinv;
-    const T fourthirds = T(4) / T(3);
-    const T g = ld(C.gamma, s), gm = ld(C.gamma, s + n.om[D]);
-    return a + (fourthirds * be + g + fourthirds * bm + gm + E1 + E1p + E2 + E2p) * dxsqinv;
-}
-
-// ------------------------------------------------------------ face arithmetic on values
-// L phi of one 3D face of component D from its loaded operands: p0 and nb =
-// {+x, -x, +y, -y, +z, -z} of the own component, q1/q2 the cross terms
-// {q(s+t), q(s), q(s-d+t), q(s-d)} of components t1, t2, a = theta alpha,
-// be/bm = beta at s and s-d, E1/E1p and E2/E2p the two edge arrays at s and
-// s+t, g/gm = gamma at s and s-d; b, c the constant beta, gamma of |visc|
-// 1..3.  Same expressions, same order as face_L3_own.
-template <class T, int VISC>
-__device__ __forceinline__ T face_L3_vals(T p0, const T (&nb)[6], int D, const T (&q1)[4], const T (&q2)[4], T a, T be, T bm,
-                                          T E1, T E1p, T E2, T E2p, T g, T gm, T dxsqinv, T b, T c) {
-    const T onethird = T(1) / T(3), twothirds = T(2) / T(3), fourthirds = T(4) / T(3);
-    if (VISC == 1) {
-        T nbs = nb[0] + nb[1] + nb[2] + nb[3] + nb[4] + nb[5];
-        return p0 * (a + T(6) * b * dxsqinv) - nbs * b * dxsqinv;
-    }
-    const int t1 = (D == 0) ? 1 : 0, t2 = (D == 2) ? 1 : 2;
-    const T ppd = nb[2 * D], pmd = nb[2 * D + 1];
-    const T pp1 = nb[2 * t1], pm1 = nb[2 * t1 + 1];
-    const T pp2 = nb[2 * t2], pm2 = nb[2 * t2 + 1];
-    const T c10 = q1[0], c11 = q1[1], c12 = q1[2], c13 = q1[3];
-    const T c20 = q2[0], c21 = q2[1], c22 = q2[2], c23 = q2[3];
-    if (VISC == 2) {
-        return p0 * (a + T(8) * b * dxsqinv) -
-               (T(2) * ppd + T(2) * pmd + pp1 + pm1 + pp2 + pm2 + c10 - c11 - c12 + c13 + c20 - c21 - c22 + c23) * b * dxsqinv;
-    }
-    if (VISC == 3) {
-        const T nbt = pp1 + pm1 + pp2 + pm2;
-        return p0 * (a + (T(20) * b * onethird + T(2) * c) * dxsqinv) -
-               ((ppd + pmd) * (fourthirds * b + c) + nbt * b +
-                (c10 - c11 - c12 + c13 + c20 - c21 - c22 + c23) * (onethird * b + c)) * dxsqinv;
-    }
-    if (VISC == -1) {
-        return p0 * (a + (be + bm + E1 + E1p + E2 + E2p) * dxsqinv) -
-               (ppd * be + pmd * bm + pp1 * E1p + pm1 * E1 + pp2 * E2p + pm2 * E2) * dxsqinv;
-    }
-    if (VISC == -2) {
-        return p0 * (a + (T(2) * be + T(2) * bm + E1 + E1p + E2 + E2p) * dxsqinv) -
-               (T(2) * ppd * be + T(2) * pmd * bm + pp1 * E1p + pm1 * E1 + pp2 * E2p + pm2 * E2 + c10 * E1p - c11 * E1 - c12 * E1p +
-                c13 * E1 + c20 * E2p - c21 * E2 - c22 * E2p + c23 * E2) * dxsqinv;
-    }
-    // VISC == -3
-    return p0 * (a + (fourthirds * be + g + fourthirds * bm + gm + E1 + E1p + E2 + E2p) * dxsqinv) -
-           (ppd * (fourthirds * be + g) + pmd * (fourthirds * bm + gm) + pp1 * E1p + pm1 * E1 + pp2 * E2p + pm2 * E2 +
-            c10 * (E1p - twothirds * be + g) - c11 * (E1 - twothirds * be + g) - c12 * (E1p - twothirds * bm + gm) +
-            c13 * (E1 - twothirds * bm + gm) + c20 * (E2p - twothirds * be + g) - c21 * (E2 - twothirds * be + g) -
-            c22 * (E2p - twothirds * bm + gm) + c23 * (E2 - twothirds * bm + gm)) * dxsqinv;
-}
-
-// the diagonal of the same face (face_diag3's expressions)
+// Operands of one 3D face of component D with transverse directions t1 < t2:
+// p0 the face, {ppd, pmd, pp1, pm1, pp2, pm2} its own component at +-d,
+// +-t1, +-t2, q1/q2 the cross terms {q(s+t), q(s), q(s-d+t), q(s-d)} of
+// components t1, t2, a = theta alpha, be/bm = beta at s and s-d, E1/E1p and
+// E2/E2p the two edge arrays at s and s+t, g/gm = gamma at s and s-d; b, c
+// the constant beta, gamma of visc_type 1..3.
+//
+// the diagonal of stag_mg_update (stag_mg_solver.f90:1637-2463); for every
+// visc_type but 3 also the factor of p0 in L phi
 template <class T, int VISC>
 __device__ __forceinline__ T face_diag3_vals(T a, T be, T bm, T E1, T E1p, T E2, T E2p, T g, T gm, T dxsqinv, T b, T c) {
     if (VISC == 1) return a + T(6) * b * dxsqinv;
@@ -454,118 +323,315 @@ __device__ __forceinline__ T face_diag3_vals(T a, T be, T bm, T E1, T E1p, T E2,
     const T fourthirds = T(4) / T(3);
     return a + (fourthirds * be + g + fourthirds * bm + gm + E1 + E1p + E2 + E2p) * dxsqinv;
 }
+// the factor of p0 in L phi (diag: face_diag3_vals of the same face)
+template <class T, int VISC>
+__device__ __forceinline__ T face_centre3_vals(T diag, T a, T dxsqinv, T b, T c) {
+    if (VISC == 3) {
+        const T onethird = T(1) / T(3);
+        return a + (T(20) * b * onethird + T(2) * c) * dxsqinv;
+    }
+    return diag;
+}
+// L phi of the face (stag_applyop.f90:204-1067) with p0's factor `centre`
+template <class T, int VISC>
+__device__ __forceinline__ T face_L3_sum(T centre, T p0, const T (&nb)[6], int D, const T (&q1)[4], const T (&q2)[4], T be, T bm,
+                                         T E1, T E1p, T E2, T E2p, T g, T gm, T dxsqinv, T b, T c) {
+    const T onethird = T(1) / T(3), twothirds = T(2) / T(3), fourthirds = T(4) / T(3);
+    if (VISC == 1) {
+        T nbs = nb[0] + nb[1] + nb[2] + nb[3] + nb[4] + nb[5];
+        return p0 * centre - nbs * b * dxsqinv;
+    }
+    const int t1 = (D == 0) ? 1 : 0, t2 = (D == 2) ? 1 : 2;
+    const T ppd = nb[2 * D], pmd = nb[2 * D + 1];
+    const T pp1 = nb[2 * t1], pm1 = nb[2 * t1 + 1];
+    const T pp2 = nb[2 * t2], pm2 = nb[2 * t2 + 1];
+    const T c10 = q1[0], c11 = q1[1], c12 = q1[2], c13 = q1[3];
+    const T c20 = q2[0], c21 = q2[1], c22 = q2[2], c23 = q2[3];
+    if (VISC == 2) {
+        return p0 * centre -
+               (T(2) * ppd + T(2) * pmd + pp1 + pm1 + pp2 + pm2 + c10 - c11 - c12 + c13 + c20 - c21 - c22 + c23) * b * dxsqinv;
+    }
+    if (VISC == 3) {
+        const T nbt = pp1 + pm1 + pp2 + pm2;
+        return p0 * centre -
+               ((ppd + pmd) * (fourthirds * b + c) + nbt * b +
+                (c10 - c11 - c12 + c13 + c20 - c21 - c22 + c23) * (onethird * b + c)) * dxsqinv;
+    }
+    if (VISC == -1) {
+        return p0 * centre - (ppd * be + pmd * bm + pp1 * E1p + pm1 * E1 + pp2 * E2p + pm2 * E2) * dxsqinv;
+    }
+    if (VISC == -2) {
+        return p0 * centre -
+               (T(2) * ppd * be + T(2) * pmd * bm + pp1 * E1p + pm1 * E1 + pp2 * E2p + pm2 * E2 + c10 * E1p - c11 * E1 - c12 * E1p +
+                c13 * E1 + c20 * E2p - c21 * E2 - c22 * E2p + c23 * E2) * dxsqinv;
+    }
+    // VISC == -3
+    return p0 * centre -
+           (ppd * (fourthirds * be + g) + pmd * (fourthirds * bm + gm) + pp1 * E1p + pm1 * E1 + pp2 * E2p + pm2 * E2 +
+            c10 * (E1p - twothirds * be + g) - c11 * (E1 - twothirds * be + g) - c12 * (E1p - twothirds * bm + gm) +
+            c13 * (E1 - twothirds * bm + gm) + c20 * (E2p - twothirds * be + g) - c21 * (E2 - twothirds * be + g) -
+            c22 * (E2p - twothirds * bm + gm) + c23 * (E2 - twothirds * bm + gm)) * dxsqinv;
+}
+template <class T, int VISC>
+__device__ __forceinline__ T face_L3_vals(T p0, const T (&nb)[6], int D, const T (&q1)[4], const T (&q2)[4], T a, T be, T bm,
+                                          T E1, T E1p, T E2, T E2p, T g, T gm, T dxsqinv, T b, T c) {
+    const T diag = face_diag3_vals<T, VISC>(a, be, bm, E1, E1p, E2, E2p, g, gm, dxsqinv, b, c);
+    const T centre = face_centre3_vals<T, VISC>(diag, a, dxsqinv, b, c);
+    return face_L3_sum<T, VISC>(centre, p0, nb, D, q1, q2, be, bm, E1, E1p, E2, E2p, g, gm, dxsqinv, b, c);
+}
+// one Gauss-Seidel update from its pieces (stag_mg_update)
+template <class T>
+__device__ __forceinline__ T gs_update(T p0, T omega, T rhs, T Lp, T diag) {
+    return p0 + omega * (rhs - Lp) / diag;
+}
 
-// One Gauss-Seidel update of a 3D face of component D on a periodic grid,
-// phi + omega (rhs - L phi) / diag, with every operand read once from
-// global memory and L phi and the diagonal formed from the same values
-// (face_L3_vals, face_diag3_vals: face_L3 / face_diag3's expressions, so
-// the same bits).
-template <class T, int VISC, int D>
-__device__ __forceinline__ T face_update3(const T* const phi[3], const Coef<T>& C, const T* rhs, const Nb& n, T dxsqinv, T b,
-                                          T c, T omega) {
+// the coefficients of a 3D face
+template <class T>
+struct FaceCoef3 {
+    T a, be, bm, E1, E1p, E2, E2p, g, gm;
+};
+template <class T, int VISC, int D, bool W = false>
+__device__ __forceinline__ FaceCoef3<T> face_coef3(const Coef<T>& C, const Nb& n) {
     constexpr int t1 = Perm3<D>::t1, t2 = Perm3<D>::t2, e1 = Perm3<D>::e1, e2 = Perm3<D>::e2;
     const int s = n.s;
-    const T* p = phi[D];
-    const T p0 = ld(p, s);
-    const T nb[6] = {ld(p, s + n.op[0]), ld(p, s + n.om[0]), ld(p, s + n.op[1]),
-                     ld(p, s + n.om[1]), ld(p, s + n.op[2]), ld(p, s + n.om[2])};
-    T q1[4] = {T(0), T(0), T(0), T(0)}, q2[4] = {T(0), T(0), T(0), T(0)};
-    if constexpr (VISC == 2 || VISC == 3 || VISC == -2 || VISC == -3) {
-        const T* a1 = phi[t1];
-        const T* a2 = phi[t2];
-        q1[0] = ld(a1, s + n.op[t1]);
-        q1[1] = ld(a1, s);
-        q1[2] = ld(a1, s + n.om[D] + n.op[t1]);
-        q1[3] = ld(a1, s + n.om[D]);
-        q2[0] = ld(a2, s + n.op[t2]);
-        q2[1] = ld(a2, s);
-        q2[2] = ld(a2, s + n.om[D] + n.op[t2]);
-        q2[3] = ld(a2, s + n.om[D]);
-    }
-    const T a = alpha_at(C, D, s);
-    T be = T(0), bm = T(0), E1 = T(0), E1p = T(0), E2 = T(0), E2p = T(0), g = T(0), gm = T(0);
+    FaceCoef3<T> k{};
+    k.a = alpha_at(C, D, s);
     if constexpr (VISC < 0) {
-        be = ld(C.beta, s);
-        bm = ld(C.beta, s + n.om[D]);
-        E1 = ld(C.bed[e1], s);
-        E1p = ld(C.bed[e1], s + n.op[t1]);
-        E2 = ld(C.bed[e2], s);
-        E2p = ld(C.bed[e2], s + n.op[t2]);
+        k.be = ld(C.beta, s);
+        k.bm = ld(C.beta, s + n.om[D]);
+        k.E1 = ld(C.bed[e1], W ? edge_at(n, e1, -1) : s);
+        k.E1p = ld(C.bed[e1], W ? edge_at(n, e1, t1) : s + n.op[t1]);
+        k.E2 = ld(C.bed[e2], W ? edge_at(n, e2, -1) : s);
+        k.E2p = ld(C.bed[e2], W ? edge_at(n, e2, t2) : s + n.op[t2]);
     }
     if constexpr (VISC == -3) {
-        g = ld(C.gamma, s);
-        gm = ld(C.gamma, s + n.om[D]);
+        k.g = ld(C.gamma, s);
+        k.gm = ld(C.gamma, s + n.om[D]);
     }
-    const T Lp = face_L3_vals<T, VISC>(p0, nb, D, q1, q2, a, be, bm, E1, E1p, E2, E2p, g, gm, dxsqinv, b, c);
-    const T fac = face_diag3_vals<T, VISC>(a, be, bm, E1, E1p, E2, E2p, g, gm, dxsqinv, b, c);
-    return p0 + omega * (ld(rhs, s) - Lp) / fac;
+    return k;
+}
+// the cross terms of a 3D face read through phi
+template <class T, int VISC, int D, int LD = 0, class TP = T, bool W = false>
+__device__ __forceinline__ void face_cross3(const TP* const phi[3], const Nb& n, T (&q1)[4], T (&q2)[4]) {
+    constexpr int t1 = Perm3<D>::t1, t2 = Perm3<D>::t2;
+    const int s = n.s;
+    if constexpr (VISC == 1 || VISC == -1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) q1[q] = q2[q] = T(0);
+        return;
+    }
+    const TP* a1 = phi[t1];
+    const TP* a2 = phi[t2];
+    q1[0] = (T)ldp<LD>(a1, s + n.op[t1]);
+    q1[1] = (T)ldp<LD>(a1, s);
+    q1[2] = (T)ldp<LD>(a1, s + n.om[D] + n.op[t1]);
+    q1[3] = (T)ldp<LD>(a1, s + n.om[D]);
+    q2[0] = (T)ldp<LD>(a2, s + n.op[t2]);
+    q2[1] = (T)ldp<LD>(a2, s);
+    q2[2] = (T)ldp<LD>(a2, s + n.om[D] + n.op[t2]);
+    q2[3] = (T)ldp<LD>(a2, s + n.om[D]);
+    if constexpr (W) {
+        // component t across its own wall at +t is zero (the face is not a wall face, so -d stays inside)
+        const int m1 = wall_mul(n, t1, t1, true), m2 = wall_mul(n, t2, t2, true);
+        q1[0] = wapply(m1, q1[0]);
+        q1[2] = wapply(m1, q1[2]);
+        q2[0] = wapply(m2, q2[0]);
+        q2[2] = wapply(m2, q2[2]);
+    }
+}
+// the six own neighbours of a 3D face of component D, {+x, -x, +y, -y, +z, -z}
+template <class T, int D, int LD = 0, class TP = T, bool W = false>
+__device__ __forceinline__ void face_own3(const TP* p, const Nb& n, T (&nb)[6]) {
+    const int s = n.s;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        nb[2 * d] = (T)ldp<LD>(p, s + n.op[d]);
+        nb[2 * d + 1] = (T)ldp<LD>(p, s + n.om[d]);
+        if constexpr (W) {
+            nb[2 * d] = wapply(wall_mul(n, D, d, true), nb[2 * d]);
+            nb[2 * d + 1] = wapply(wall_mul(n, D, d, false), nb[2 * d + 1]);
+        }
+    }
+}
+
+// The face value with the own component's centre p0 and its six neighbours
+// nb = {+x, -x, +y, -y, +z, -z} supplied by the caller (global memory for the
+// plain kernels, shared memory for the fused red/black pair); the other two
+// components and the coefficients are read through phi / C.
+template <class T, int VISC, int D, int LD = 0, class TP = T, bool W = false>
+__device__ __forceinline__ T face_L3_own(const T p0, const T (&nb)[6], const TP* const phi[3], const Coef<T>& C, const Nb& n,
+                                         T dxsqinv, T b, T c) {
+    const FaceCoef3<T> k = face_coef3<T, VISC, D, W>(C, n);
+    T q1[4], q2[4];
+    face_cross3<T, VISC, D, LD, TP, W>(phi, n, q1, q2);
+    return face_L3_vals<T, VISC>(p0, nb, D, q1, q2, k.a, k.be, k.bm, k.E1, k.E1p, k.E2, k.E2p, k.g, k.gm, dxsqinv, b, c);
+}
+
+template <class T, int VISC, int D, int LD = 0, class TP = T, bool W = false>
+__device__ __forceinline__ T face_L3(const TP* const phi[3], const Coef<T>& C, const Nb& n, T dxsqinv, T b, T c) {
+    const T p0 = (T)ldp<LD>(phi[D], n.s);
+    T nb[6];
+    face_own3<T, D, LD, TP, W>(phi[D], n, nb);
+    return face_L3_own<T, VISC, D, LD, TP, W>(p0, nb, phi, C, n, dxsqinv, b, c);
+}
+
+template <class T, int VISC, int D, bool W = false>
+__device__ __forceinline__ T face_diag3(const Coef<T>& C, const Nb& n, T dxsqinv, T b, T c) {
+    const FaceCoef3<T> k = face_coef3<T, VISC, D, W>(C, n);
+    return face_diag3_vals<T, VISC>(k.a, k.be, k.bm, k.E1, k.E1p, k.E2, k.E2p, k.g, k.gm, dxsqinv, b, c);
+}
+
+// One Gauss-Seidel update of a 3D face of component D,
+// phi + omega (rhs - L phi) / diag, with every operand read once and L phi
+// and the diagonal formed from the same values.
+template <class T, int VISC, int D, int LD = 0, bool W = false>
+__device__ __forceinline__ T face_update3(const T* const phi[3], const Coef<T>& C, const T* rhs, const Nb& n, T dxsqinv, T b,
+                                          T c, T omega) {
+    const T p0 = ldp<LD>(phi[D], n.s);
+    T nb[6], q1[4], q2[4];
+    face_own3<T, D, LD, T, W>(phi[D], n, nb);
+    face_cross3<T, VISC, D, LD, T, W>(phi, n, q1, q2);
+    const FaceCoef3<T> k = face_coef3<T, VISC, D, W>(C, n);
+    const T diag = face_diag3_vals<T, VISC>(k.a, k.be, k.bm, k.E1, k.E1p, k.E2, k.E2p, k.g, k.gm, dxsqinv, b, c);
+    const T centre = face_centre3_vals<T, VISC>(diag, k.a, dxsqinv, b, c);
+    const T Lp = face_L3_sum<T, VISC>(centre, p0, nb, D, q1, q2, k.be, k.bm, k.E1, k.E1p, k.E2, k.E2p, k.g, k.gm, dxsqinv, b, c);
+    return gs_update(p0, omega, ldp<LD>(rhs, n.s), Lp, diag);
 }
 
 // ------------------------------------------------------------------ 2D
-template <class T, int VISC, int D, int LD = 0, class TP = T, bool W = false>
-__device__ __forceinline__ T face_L2(const TP* const phi[3], const Coef<T>& C, const Nb& n, T dxsqinv, T b, T c) {
+// Operands as in 3D with one transverse direction t: {ppd, pmd, ppt, pmt}
+// the own component at +-d, +-t, q the cross terms, E/Ep the nodal array at
+// s and s+t.
+template <class T>
+struct FaceCoef2 {
+    T a, be, bm, E, Ep, g, gm;
+};
+template <class T, int VISC, int D, bool W = false>
+__device__ __forceinline__ FaceCoef2<T> face_coef2(const Coef<T>& C, const Nb& n) {
     constexpr int t = 1 - D;
+    const int s = n.s;
+    FaceCoef2<T> k{};
+    k.a = alpha_at(C, D, s);
+    if constexpr (VISC < 0) {
+        k.be = ld(C.beta, s);
+        k.bm = ld(C.beta, s + n.om[D]);
+        k.E = ld(C.bed[0], W ? edge_at(n, 0, -1) : s);
+        k.Ep = ld(C.bed[0], W ? edge_at(n, 0, t) : s + n.op[t]);
+    }
+    if constexpr (VISC == -3) {
+        k.g = ld(C.gamma, s);
+        k.gm = ld(C.gamma, s + n.om[D]);
+    }
+    return k;
+}
+// the diagonal of stag_mg_update
+template <class T, int VISC>
+__device__ __forceinline__ T face_diag2_vals(const FaceCoef2<T>& k, T dxsqinv, T b, T c) {
+    if (VISC == 1) return k.a + T(4) * b * dxsqinv;
+    if (VISC == 2) return k.a + T(6) * b * dxsqinv;
+    if (VISC == 3) return k.a + (T(14) / T(3) * b + T(2) * c) * dxsqinv;
+    if (VISC == -1) return k.a + (k.be + k.bm + k.E + k.Ep) * dxsqinv;
+    if (VISC == -2) return k.a + (T(2) * k.be + T(2) * k.bm + k.E + k.Ep) * dxsqinv;
+    const T fourthirds = T(4) / T(3);
+    return k.a + (fourthirds * k.be + k.g + fourthirds * k.bm + k.gm + k.E + k.Ep) * dxsqinv;
+}
+// p0's factor in L phi: the Fortran adds the two edge values the other way
+// round there for the variable-coefficient operators
+template <class T, int VISC>
+__device__ __forceinline__ T face_centre2_vals(const FaceCoef2<T>& k, T dxsqinv, T b, T c) {
+    if (VISC == 1 || VISC == 2) return face_diag2_vals<T, VISC>(k, dxsqinv, b, c);
+    const T onethird = T(1) / T(3), fourthirds = T(4) / T(3);
+    if (VISC == 3) return k.a + (T(14) * b * onethird + T(2) * c) * dxsqinv;
+    if (VISC == -1) return k.a + (k.be + k.bm + k.Ep + k.E) * dxsqinv;
+    if (VISC == -2) return k.a + (T(2) * k.be + T(2) * k.bm + k.Ep + k.E) * dxsqinv;
+    return k.a + (fourthirds * k.be + k.g + fourthirds * k.bm + k.gm + k.Ep + k.E) * dxsqinv;
+}
+template <class T, int VISC>
+__device__ __forceinline__ T face_L2_sum(T centre, T p0, T ppd, T pmd, T ppt, T pmt, const T (&q)[4], const FaceCoef2<T>& k,
+                                         T dxsqinv, T b, T c) {
     const T onethird = T(1) / T(3), twothirds = T(2) / T(3), fourthirds = T(4) / T(3);
+    const T be = k.be, bm = k.bm, E = k.E, Ep = k.Ep, g = k.g, gm = k.gm;
+    // x: i+1, i-1, j+1, j-1 ; y: j+1, j-1, i+1, i-1  (own direction first)
+    if (VISC == 1) return p0 * centre - (ppd + pmd + ppt + pmt) * b * dxsqinv;
+    if (VISC == 2) return p0 * centre - (T(2) * ppd + T(2) * pmd + ppt + pmt + q[0] - q[1] - q[2] + q[3]) * b * dxsqinv;
+    if (VISC == 3) {
+        return p0 * centre -
+               ((ppd + pmd) * (fourthirds * b + c) + (ppt + pmt) * b + (q[0] - q[1] - q[2] + q[3]) * (onethird * b + c)) * dxsqinv;
+    }
+    if (VISC == -1) return p0 * centre - (ppd * be + pmd * bm + ppt * Ep + pmt * E) * dxsqinv;
+    if (VISC == -2) {
+        return p0 * centre -
+               (T(2) * ppd * be + T(2) * pmd * bm + ppt * Ep + pmt * E + q[0] * Ep - q[1] * E - q[2] * Ep + q[3] * E) * dxsqinv;
+    }
+    return p0 * centre -
+           (ppd * (fourthirds * be + g) + pmd * (fourthirds * bm + gm) + ppt * Ep + pmt * E + q[0] * (Ep - twothirds * be + g) -
+            q[1] * (E - twothirds * be + g) - q[2] * (Ep - twothirds * bm + gm) + q[3] * (E - twothirds * bm + gm)) * dxsqinv;
+}
+// own neighbours {+d, -d, +t, -t} and cross terms of a 2D face
+template <class T, int VISC, int D, int LD = 0, class TP = T, bool W = false>
+__device__ __forceinline__ void face_phi2(const TP* const phi[3], const Nb& n, T (&nb)[4], T (&x)[4]) {
+    constexpr int t = 1 - D;
     const TP* p = phi[D];
     const TP* q = phi[t];
     const int s = n.s;
-    const T p0 = (T)ldp<LD>(p, s);
-    const T a = alpha_at(C, D, s);
-    T ppd = (T)ldp<LD>(p, s + n.op[D]), pmd = (T)ldp<LD>(p, s + n.om[D]);
-    T ppt = (T)ldp<LD>(p, s + n.op[t]), pmt = (T)ldp<LD>(p, s + n.om[t]);
+    nb[0] = (T)ldp<LD>(p, s + n.op[D]);
+    nb[1] = (T)ldp<LD>(p, s + n.om[D]);
+    nb[2] = (T)ldp<LD>(p, s + n.op[t]);
+    nb[3] = (T)ldp<LD>(p, s + n.om[t]);
     if constexpr (W) {
-        ppd = wapply(wall_mul(n, D, D, true), ppd);
-        pmd = wapply(wall_mul(n, D, D, false), pmd);
-        ppt = wapply(wall_mul(n, D, t, true), ppt);
-        pmt = wapply(wall_mul(n, D, t, false), pmt);
+        nb[0] = wapply(wall_mul(n, D, D, true), nb[0]);
+        nb[1] = wapply(wall_mul(n, D, D, false), nb[1]);
+        nb[2] = wapply(wall_mul(n, D, t, true), nb[2]);
+        nb[3] = wapply(wall_mul(n, D, t, false), nb[3]);
     }
-    if (VISC == 1) {
-        // x: i+1, i-1, j+1, j-1 ; y: j+1, j-1, i+1, i-1  (own direction first)
-        return p0 * (a + T(4) * b * dxsqinv) - (ppd + pmd + ppt + pmt) * b * dxsqinv;
+    if constexpr (VISC == 1 || VISC == -1) {
+        x[0] = x[1] = x[2] = x[3] = T(0);
+    } else {
+        x[0] = (T)ldp<LD>(q, s + n.op[t]);
+        x[1] = (T)ldp<LD>(q, s);
+        x[2] = (T)ldp<LD>(q, s + n.om[D] + n.op[t]);
+        x[3] = (T)ldp<LD>(q, s + n.om[D]);
+        if constexpr (W) {
+            const int m = wall_mul(n, t, t, true);
+            x[0] = wapply(m, x[0]);
+            x[2] = wapply(m, x[2]);
+        }
     }
-    T c0 = (T)ldp<LD>(q, s + n.op[t]), c1 = (T)ldp<LD>(q, s), c2 = (T)ldp<LD>(q, s + n.om[D] + n.op[t]), c3 = (T)ldp<LD>(q, s + n.om[D]);
-    if constexpr (W) {
-        const int m = wall_mul(n, t, t, true);
-        c0 = wapply(m, c0);
-        c2 = wapply(m, c2);
-    }
-    if (VISC == 2) {
-        return p0 * (a + T(6) * b * dxsqinv) - (T(2) * ppd + T(2) * pmd + ppt + pmt + c0 - c1 - c2 + c3) * b * dxsqinv;
-    }
-    if (VISC == 3) {
-        return p0 * (a + (T(14) * b * onethird + T(2) * c) * dxsqinv) -
-               ((ppd + pmd) * (fourthirds * b + c) + (ppt + pmt) * b + (c0 - c1 - c2 + c3) * (onethird * b + c)) * dxsqinv;
-    }
-    const T be = ld(C.beta, s), bm = ld(C.beta, s + n.om[D]);
-    const T E = ld(C.bed[0], W ? edge_at(n, 0, -1) : s), Ep = ld(C.bed[0], W ? edge_at(n, 0, t) : s + n.op[t]);
-    if (VISC == -1) {
-        return p0 * (a + (be + bm + Ep + E) * dxsqinv) - (ppd * be + pmd * bm + ppt * Ep + pmt * E) * dxsqinv;
-    }
-    if (VISC == -2) {
-        return p0 * (a + (T(2) * be + T(2) * bm + Ep + E) * dxsqinv) -
-               (T(2) * ppd * be + T(2) * pmd * bm + ppt * Ep + pmt * E + c0 * Ep - c1 * E - c2 * Ep + c3 * E) * dxsqinv;
-    }
-    const T g = ld(C.gamma, s), gm = ld(C.gamma, s + n.om[D]);
-    return p0 * (a + (fourthirds * be + g + fourthirds * bm + gm + Ep + E) * dxsqinv) -
-           (ppd * (fourthirds * be + g) + pmd * (fourthirds * bm + gm) + ppt * Ep + pmt * E + c0 * (Ep - twothirds * be + g) -
-            c1 * (E - twothirds * be + g) - c2 * (Ep - twothirds * bm + gm) + c3 * (E - twothirds * bm + gm)) * dxsqinv;
+}
+template <class T, int VISC, int D, int LD = 0, class TP = T, bool W = false>
+__device__ __forceinline__ T face_L2(const TP* const phi[3], const Coef<T>& C, const Nb& n, T dxsqinv, T b, T c) {
+    T nb[4], x[4];
+    face_phi2<T, VISC, D, LD, TP, W>(phi, n, nb, x);
+    const FaceCoef2<T> k = face_coef2<T, VISC, D, W>(C, n);
+    return face_L2_sum<T, VISC>(face_centre2_vals<T, VISC>(k, dxsqinv, b, c), (T)ldp<LD>(phi[D], n.s), nb[0], nb[1], nb[2], nb[3], x,
+                                k, dxsqinv, b, c);
 }
 
 template <class T, int VISC, int D, bool W = false>
 __device__ __forceinline__ T face_diag2(const Coef<T>& C, const Nb& n, T dxsqinv, T b, T c) {
-    constexpr int t = 1 - D;
-    const int s = n.s;
-    const T a = alpha_at(C, D, s);
-    if (VISC == 1) return a + T(4) * b * dxsqinv;
-    if (VISC == 2) return a + T(6) * b * dxsqinv;
-    if (VISC == 3) return a + (T(14) / T(3) * b + T(2) * c) * dxsqinv;
-    const T be = ld(C.beta, s), bm = ld(C.beta, s + n.om[D]);
-    const T E = ld(C.bed[0], W ? edge_at(n, 0, -1) : s), Ep = ld(C.bed[0], W ? edge_at(n, 0, t) : s + n.op[t]);
-    if (VISC == -1) return a + (be + bm + E + Ep) * dxsqinv;
-    if (VISC == -2) return a + (T(2) * be + T(2) * bm + E + Ep) * dxsqinv;
-    const T fourthirds = T(4) / T(3);
-    const T g = ld(C.gamma, s), gm = ld(C.gamma, s + n.om[D]);
-    return a + (fourthirds * be + g + fourthirds * bm + gm + E + Ep) * dxsqinv;
+    return face_diag2_vals<T, VISC>(face_coef2<T, VISC, D, W>(C, n), dxsqinv, b, c);
+}
+
+// one Gauss-Seidel update of a 2D face (face_update3's counterpart)
+template <class T, int VISC, int D, int LD = 0, bool W = false>
+__device__ __forceinline__ T face_update2(const T* const phi[3], const Coef<T>& C, const T* rhs, const Nb& n, T dxsqinv, T b,
+                                          T c, T omega) {
+    T nb[4], x[4];
+    face_phi2<T, VISC, D, LD, T, W>(phi, n, nb, x);
+    const FaceCoef2<T> k = face_coef2<T, VISC, D, W>(C, n);
+    const T p0 = ldp<LD>(phi[D], n.s);
+    const T Lp = face_L2_sum<T, VISC>(face_centre2_vals<T, VISC>(k, dxsqinv, b, c), p0, nb[0], nb[1], nb[2], nb[3], x, k, dxsqinv,
+                                      b, c);
+    return gs_update(p0, omega, ldp<LD>(rhs, n.s), Lp, face_diag2_vals<T, VISC>(k, dxsqinv, b, c));
+}
+
+template <class T, int DM, int VISC, int D, int LD = 0, bool W = false>
+__device__ __forceinline__ T face_update(const T* const phi[3], const Coef<T>& C, const T* rhs, const Nb& n, T dxsqinv, T b, T c,
+                                         T omega) {
+    if constexpr (DM == 2)
+        return face_update2<T, VISC, D, LD, W>(phi, C, rhs, n, dxsqinv, b, c, omega);
+    else
+        return face_update3<T, VISC, D, LD, W>(phi, C, rhs, n, dxsqinv, b, c, omega);
 }
 
 template <class T, int DM, int VISC, int D, int LD = 0, class TP = T, bool W = false>
