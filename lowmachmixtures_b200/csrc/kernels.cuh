@@ -65,6 +65,18 @@ static inline G3 geom3_tuned(int kernel, int wbytes, int visc, const Dims& D, in
     return s.bx ? geom3_shape(nx, ny, nz, s) : geom3(nx, ny, nz);
 }
 
+// two consecutive entries
+template <class T>
+struct Pair2;
+template <>
+struct Pair2<double> {
+    using type = double2;
+};
+template <>
+struct Pair2<float> {
+    using type = float2;
+};
+
 // --------------------------------------------------------------- applyop
 // W: a grid with walls; L phi is zero on the wall faces (stag_applyop.f90:197-201)
 template <class T, int DM, int VISC, bool W = false>
@@ -187,6 +199,37 @@ __global__ void __launch_bounds__(kThreads) k_gs_colour(Dims D, Coef<T> C, const
     const T b = ld(C.beta, 0), c = ld(C.gamma, 0);
     T* p = (COMP == 0) ? p0 : (COMP == 1 ? p1 : p2);
     p[nb.s] = face_update<T, DM, VISC, COMP, 0, W>(phi, C, rhs, nb, dxsqinv, b, c, omega);
+}
+
+// The first colour of a smooth that starts from phi = 0 (every V-cycle's way
+// down): L phi is zero, so the colour is omega rhs / diag, and the same launch
+// writes the zeros of every other face of the level -- phi needs no memset
+// before and no load here.  One thread per pair of faces of a row, 2-entry
+// stores (even levels; every field starts on a pair: its base is 256-byte
+// aligned or an even number of entries past one that is).
+template <class T, int DM, int VISC, bool W = false>
+__global__ void __launch_bounds__(kThreads) k_gs_zero(Dims D, Coef<T> C, const T* __restrict__ rhs, T* __restrict__ p0, T* __restrict__ p1,
+                                                      T* __restrict__ p2, T omega, T dxsqinv) {
+    const Pos q = pos3(D.nx >> 1, D.ny);
+    if (!q.ok) {
+        pdl_enter();
+        return;
+    }
+    const int j = q.j, k = q.k, odd = (j + ck<DM>(k)) & 1;
+    Nb nb = W ? make_nbw(D, 2 * q.i + odd, j, k) : make_nb(D, 2 * q.i + odd, j, k);
+    const T diag = face_diag<T, DM, VISC, 0, W>(C, nb, dxsqinv, ld(C.beta, 0), ld(C.gamma, 0));
+    pdl_enter();
+    T v = T(0);
+    if (!(W && wall_face(nb, 0))) v = gs_update(T(0), omega, ld(rhs, nb.s), T(0), diag);
+    using V2 = typename Pair2<T>::type;
+    const int t = q.i + (D.nx >> 1) * (j + D.ny * k);
+    V2 x, z;
+    x.x = odd ? T(0) : v;
+    x.y = odd ? v : T(0);
+    z.x = z.y = T(0);
+    reinterpret_cast<V2*>(p0)[t] = x;
+    reinterpret_cast<V2*>(p1)[t] = z;
+    if constexpr (DM == 3) reinterpret_cast<V2*>(p2)[t] = z;
 }
 
 // --------------------------------------------------------------- odd levels
@@ -757,6 +800,31 @@ __global__ void __launch_bounds__(kThreads) k_cc_smooth(Dims D, const T* a0, con
     phi[nb.s] = cc_update<T, DM, U>(a, cu, phi, rhs, nb, dxsqinv);
 }
 
+// the first colour of a pressure smooth from phi = 0 (as k_gs_zero): red
+// cells get rhs / diag, black ones zero
+template <class T, int DM, bool U = false>
+__global__ void __launch_bounds__(kThreads) k_cc_zero(Dims D, const T* a0, const T* a1, const T* a2, const T* __restrict__ rhs,
+                                                      T* __restrict__ phi, T dxsqinv, T cu) {
+    const Pos q = pos3(D.nx >> 1, D.ny);
+    if (!q.ok) {
+        pdl_enter();
+        return;
+    }
+    const int j = q.j, k = q.k, odd = (j + ck<DM>(k)) & 1;
+    const Nb nb = make_nb(D, 2 * q.i + odd, j, k);
+    const T* a[3] = {a0, a1, a2};
+    T c[6];
+    cc_coef<T, DM, U>(a, cu, nb, c);
+    const T diag = cc_diag_vals<T, DM>(c, dxsqinv);
+    pdl_enter();
+    const T v = T(0) + ld(rhs, nb.s) / diag;
+    using V2 = typename Pair2<T>::type;
+    V2 x;
+    x.x = odd ? T(0) : v;
+    x.y = odd ? v : T(0);
+    reinterpret_cast<V2*>(phi)[q.i + (D.nx >> 1) * (j + D.ny * k)] = x;
+}
+
 // one colour of the pressure smoother on an odd level: new values from the
 // values before the colour's pass (out), then copied back
 template <class T, int DM>
@@ -928,17 +996,6 @@ static inline int reduce_pairs(const Dims& D, size_t elem, const void* const a[4
     }
     return 1;
 }
-
-template <class T>
-struct Pair2;
-template <>
-struct Pair2<double> {
-    using type = double2;
-};
-template <>
-struct Pair2<float> {
-    using type = float2;
-};
 
 // vec = 1 (reduce_pairs): entries in pairs by one 16- (FP64) or 8-byte
 // (FP32) load per array; the sums change order within a thread's pair only
@@ -1251,6 +1308,25 @@ void launch_gs_colour(const LevelDev<T>& L, int visc, int color, const T* const 
 #undef GS
 }
 
+// the first colour from phi = 0 (k_gs_zero); false: the level takes no such
+// launch (odd counts), nothing done
+template <class T>
+bool launch_gs_zero(const LevelDev<T>& L, int visc, const T* const rhs[3], T* const phi[3], double omega, cudaStream_t s) {
+    if (odd_level(L.D)) return false;
+    if (L.D.wall) {
+        wl_gs_zero<T>(L, visc, rhs, phi, omega, s);
+        return true;
+    }
+    const T dxsqinv = T(1.0 / (L.dx * L.dx)), om = (T)omega;
+    const G3 g = geom3(L.D.nx / 2, L.D.ny, L.D.nz);
+    if (L.D.dm == 2) {
+        LMM_VISC_DISPATCH(visc, launch_pdl(k_gs_zero<T, 2, V>, g.grid, g.block, 0, s, L.D, L.coef(), rhs[0], phi[0], phi[1], phi[1], om, dxsqinv))
+    } else {
+        LMM_VISC_DISPATCH(visc, launch_pdl(k_gs_zero<T, 3, V>, g.grid, g.block, 0, s, L.D, L.coef(), rhs[0], phi[0], phi[1], phi[2], om, dxsqinv))
+    }
+    return true;
+}
+
 // tile of the fused pair on one level (ok == false: use the per-colour
 // kernels); tz_req > 1 forces the planes per block
 struct PairGeom {
@@ -1406,6 +1482,21 @@ void launch_cc_smooth(const LevelDev<T>& L, int parity, cudaStream_t s, int reve
         launch_pdl(k_cc_smooth<T, 2>, g.grid, g.block, 0, s, L.D, L.pa[0], L.pa[1], L.pa[2], L.prhs, L.pphi, parity, dxsqinv, T(0), rev);
     else
         launch_pdl(k_cc_smooth<T, 3>, g.grid, g.block, 0, s, L.D, L.pa[0], L.pa[1], L.pa[2], L.prhs, L.pphi, parity, dxsqinv, T(0), rev);
+}
+
+template <class T>
+bool launch_cc_zero(const LevelDev<T>& L, cudaStream_t s) {
+    if (odd_level(L.D)) return false;
+    const T dxsqinv = T(1.0 / (L.dx * L.dx));
+    const G3 g = geom3(L.D.nx / 2, L.D.ny, L.D.nz);
+#define CZ(DM_, U_) launch_pdl(k_cc_zero<T, DM_, U_>, g.grid, g.block, 0, s, L.D, L.pa[0], L.pa[1], L.pa[2], L.prhs, L.pphi, dxsqinv, L.pa_value)
+    if (L.D.dm == 2) {
+        if (L.pa_uniform) CZ(2, true); else CZ(2, false);
+    } else {
+        if (L.pa_uniform) CZ(3, true); else CZ(3, false);
+    }
+#undef CZ
+    return true;
 }
 
 template <class T>
@@ -1568,6 +1659,8 @@ namespace lmm {
     template void launch_gs_colour<T>(const LevelDev<T>&, int, int, const T* const[3], T* const[3], double, cudaStream_t, int); \
     template void launch_jacobi<T>(const LevelDev<T>&, int, const T* const[3], const T* const[3], T* const[3], double,         \
                                    cudaStream_t);                                                                              \
+    template bool launch_gs_zero<T>(const LevelDev<T>&, int, const T* const[3], T* const[3], double, cudaStream_t);            \
+    template bool launch_cc_zero<T>(const LevelDev<T>&, cudaStream_t);                                                         \
     template bool gs_pair_supported<T>(const LevelDev<T>&, int);                                                               \
     template void launch_inverse_diag_lap<T>(const LevelDev<T>&, int, T* const[3], cudaStream_t);                                \
     template void launch_grad_mul<T>(const LevelDev<T>&, const T*, const T* const[3], T* const[3], cudaStream_t);                \

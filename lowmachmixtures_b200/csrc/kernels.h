@@ -62,6 +62,11 @@ void launch_applyop(const LevelDev<T>& L, int visc, const T* const phi[3], T* co
 template <class T>
 void launch_gs_colour(const LevelDev<T>& L, int visc, int color, const T* const rhs[3], T* const phi[3], double omega,
                       cudaStream_t s, int reverse = 0);
+// the first colour (of component x) of a smooth from phi = 0; writes every
+// face of phi, so phi's content before is not used.  false: an odd level,
+// nothing launched
+template <class T>
+bool launch_gs_zero(const LevelDev<T>& L, int visc, const T* const rhs[3], T* const phi[3], double omega, cudaStream_t s);
 // Both Gauss-Seidel colours of component comp in one launch, out of place:
 // cur[] are read, the new values of component comp go to out (3D levels with
 // even sizes; gs_pair_supported says whether the level qualifies).  kc > 0
@@ -105,6 +110,8 @@ template <class T>
 void wl_gs_colour(const LevelDev<T>& L, int visc, int color, const T* const rhs[3], T* const phi[3], double omega, cudaStream_t s,
                   int reverse = 0);
 template <class T>
+void wl_gs_zero(const LevelDev<T>& L, int visc, const T* const rhs[3], T* const phi[3], double omega, cudaStream_t s);
+template <class T>
 void wl_jacobi(const LevelDev<T>& L, int visc, const T* const rhs[3], const T* const phi_in[3], T* const phi_out[3], double omega,
                cudaStream_t s);
 template <class T>
@@ -128,6 +135,10 @@ size_t tail_smem_bytes(const LevelDev<T>* L, int nl, bool stag);
 // reverse: the launch takes the planes in decreasing order (same values)
 template <class T>
 void launch_cc_smooth(const LevelDev<T>& L, int parity, cudaStream_t s, int reverse = 0);
+// the first (red) colour of a smooth from phi = 0, writing every cell of
+// phi; false: an odd level, nothing launched
+template <class T>
+bool launch_cc_zero(const LevelDev<T>& L, cudaStream_t s);
 template <class T>
 void launch_cc_residual_restrict(const LevelDev<T>& F, const LevelDev<T>& Cc, cudaStream_t s);
 // *flag |= 1 when the level's pressure face coefficients are not all the

@@ -277,14 +277,25 @@ struct lmm_handle {
     cudaEvent_t col_ev = nullptr;   // FGMRES: the Hessenberg column has reached the host
     bool coeffs_loaded = false;
     double theta_loaded = 0.0;
-    // captured preconditioner applications: (input, output, theta, precision)
+    // captured preconditioner applications: (input, output, theta, precision, uniform_id)
     struct Graph {
         int seen = 0;
         cudaGraphExec_t exec = nullptr;
         int64_t launches = 0;
         int vcycles = 0, pvcycles = 0;
     };
-    std::map<std::tuple<const void*, const void*, double, int>, Graph> graphs;
+    std::map<std::tuple<const void*, const void*, double, int, int>, Graph> graphs;
+    // the uniform-coefficient flags and values of a coefficient load: kernel
+    // arguments of the graphs captured under it, so part of their key
+    // (uniform_id: the current one's index)
+    std::vector<std::vector<double>> uniform_states;
+    int uniform_id = 0;
+    static constexpr size_t kUniformStates = 16;
+    void drop_graphs() {
+        for (auto& kv : graphs)
+            if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+        graphs.clear();
+    }
     // learned stage (3D, FGMRES with the FP32 preconditioner): network and
     // its buffers, allocated by lmm_stokes_set_net outside the arena
     lmm_net* net = nullptr;
@@ -675,19 +686,34 @@ void load_coeffs(lmm_handle* h, const double* const alpha_dev[3], const double* 
         int* hflags = reinterpret_cast<int*>(h->hmisc + 32);
         LMM_CK(cudaMemcpyAsync(hflags, flags, 32 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
         LMM_CK(host_wait(h));
+        std::vector<double> state;
         for (int l = 0; l < (int)h->L64.size(); ++l) {
-            const bool u = l < np && hflags[l] == 0 && !h->D0.wall;
-            h->L64[l].pa_uniform = u ? 1 : 0;
-            h->L64[l].pa_value = u ? h->hmisc[l] : 0.0;
-            const bool ua = l < nv && hflags[16 + l] == 0 && h->knobs.uniform_alpha >= 0;
-            h->L64[l].a_uniform = ua ? 1 : 0;
-            h->L64[l].a_value = ua ? h->hmisc[16 + l] : 0.0;
+            LevelDev<double>& L = h->L64[l];
+            const int u = l < np && hflags[l] == 0 && !h->D0.wall;
+            const int ua = l < nv && hflags[16 + l] == 0 && h->knobs.uniform_alpha >= 0;
+            const double pv = u ? h->hmisc[l] : 0.0, av = ua ? h->hmisc[16 + l] : 0.0;
+            state.insert(state.end(), {(double)u, pv, (double)ua, av});
+            L.pa_uniform = u;
+            L.pa_value = pv;
+            L.a_uniform = ua;
+            L.a_value = av;
             if (l < (int)h->L32.size()) {
                 h->L32[l].pa_uniform = h->L64[l].pa_uniform;
                 h->L32[l].pa_value = (float)h->L64[l].pa_value;
                 h->L32[l].a_uniform = h->L64[l].a_uniform;
                 h->L32[l].a_value = (float)h->L64[l].a_value;
             }
+        }
+        auto& seen = h->uniform_states;
+        const auto it = std::find(seen.begin(), seen.end(), state);
+        h->uniform_id = (int)(it - seen.begin());
+        if (it == seen.end()) {
+            if (seen.size() >= lmm_handle::kUniformStates) {
+                h->drop_graphs();
+                seen.clear();
+                h->uniform_id = 0;
+            }
+            seen.push_back(state);
         }
     }
     h->coeffs_loaded = true;
@@ -708,8 +734,17 @@ bool use_tma_smoother(const lmm_handle* h, const LevelDev<T>& L) {
 }
 
 template <class T>
-void smooth(lmm_handle* h, LevelDev<T>& L, int nsm) {
+void zero_phi(lmm_handle* h, LevelDev<T>& L) {
+    for (int d = 0; d < h->dm; ++d) LMM_CK(cudaMemsetAsync(L.phi[d], 0, L.n * sizeof(T), h->stream));
+}
+
+// nsm smooths of one level; zero: from phi = 0, whatever phi holds
+template <class T>
+void smooth(lmm_handle* h, LevelDev<T>& L, int nsm, bool zero = false) {
     const lmm_knobs& K = h->knobs;
+    // the first colour launch writes phi where the smoother is one launch per colour
+    const bool colours = nsm > 0 && K.stag_mg_smoother != 0 && K.smoother_fusion <= 0 && !use_tma_smoother<T>(h, L);
+    if (zero && !colours) zero_phi<T>(h, L);
     if (nsm > 0 && use_tma_smoother<T>(h, L)) {
         h->tma_smoother = true;
         // TMA-staged colour pairs, ping-ponging each component between phi and tmp
@@ -753,6 +788,13 @@ void smooth(lmm_handle* h, LevelDev<T>& L, int nsm) {
             // consecutive colour launches take the planes in alternating order
             // (smoother_order = 0): each starts where the last left its operands in L2
             for (int color = 1; color <= 2 * h->dm; ++color) {
+                if (zero && m == 0 && color == 1) {
+                    if (launch_gs_zero<T>(L, K.visc_type, L.rhs, L.phi, K.stag_mg_omega, h->stream)) {
+                        check_launch();
+                        continue;
+                    }
+                    zero_phi<T>(h, L);
+                }
                 launch_gs_colour<T>(L, K.visc_type, color, L.rhs, L.phi, K.stag_mg_omega, h->stream,
                                     (K.smoother_order == 0 && color % 2 == 0) ? 1 : 0);
                 check_launch();
@@ -869,27 +911,26 @@ int tail_start(lmm_handle* h, const std::vector<LevelDev<T>>& L, int nl, bool st
     return lc;
 }
 
+// one V-cycle on L[0].phi / L[0].rhs; zero: from L[0].phi = 0, whatever the
+// array holds (the coarse levels always start from zero)
 template <class T>
-void vcycle(lmm_handle* h, std::vector<LevelDev<T>>& L) {
+void vcycle(lmm_handle* h, std::vector<LevelDev<T>>& L, bool zero = false) {
     NvtxRange nvtx_("stag_mg V-cycle");
     const lmm_knobs& K = h->knobs;
     const int nl = h->nlev;
     const int lc = tail_start<T>(h, L, nl, true);
-    // coarse-level initial guesses are zero; the tail takes those of its own levels as zero
-    for (int l = 1; l < std::min(lc, nl); ++l)
-        for (int d = 0; d < h->dm; ++d) LMM_CK(cudaMemsetAsync(L[l].phi[d], 0, L[l].n * sizeof(T), h->stream));
     for (int l = 0; l < lc && l < nl - 1; ++l) {
-        smooth<T>(h, L[l], K.stag_mg_nsmooths_down);
+        smooth<T>(h, L[l], K.stag_mg_nsmooths_down, l > 0 || zero);
         launch_residual_restrict<T>(L[l], L[l + 1], K.visc_type, L[l].rhs, L[l].phi, L[l + 1].rhs, h->stream,
                                     K.residual_fusion > 0 ? 1 : 0);
         check_launch();
     }
     if (lc < nl) {
         LMM_CK(launch_vcycle_tail<T>(&L[lc], nl - lc, K.visc_type, K.stag_mg_nsmooths_down, K.stag_mg_nsmooths_up,
-                                     K.stag_mg_nsmooths_bottom, K.stag_mg_smoother, K.stag_mg_omega, h->stream, lc > 0));
+                                     K.stag_mg_nsmooths_bottom, K.stag_mg_smoother, K.stag_mg_omega, h->stream, lc > 0 || zero));
         check_launch();
     } else {
-        smooth<T>(h, L[nl - 1], K.stag_mg_nsmooths_bottom);
+        smooth<T>(h, L[nl - 1], K.stag_mg_nsmooths_bottom, nl > 1 || zero);
     }
     for (int l = std::min(lc, nl - 1) - 1; l >= 0; --l) {
         launch_prolong_add<T>(L[l], L[l + 1], L[l + 1].phi, L[l].phi, h->stream);
@@ -923,15 +964,17 @@ void mg_resid_inf<float>(lmm_handle* h, LevelDev<float>& L0, int slot) {
     check_launch();
 }
 
-// stag_mg_solver: phi (initial guess) and rhs live in L[0].phi / L[0].rhs
+// stag_mg_solver: phi (initial guess; zero: phi = 0, whatever the array
+// holds) and rhs live in L[0].phi / L[0].rhs
 template <class T>
-void stag_mg_solver(lmm_handle* h) {
+void stag_mg_solver(lmm_handle* h, bool zero = false) {
     auto& L = levels<T>(h);
     const lmm_knobs& K = h->knobs;
     const int dm = h->dm;
     if (K.stag_mg_max_vcycles <= 1) {
-        vcycle<T>(h, L);
+        vcycle<T>(h, L, zero);
     } else {
+        if (zero) zero_phi<T>(h, L[0]);
         const int s0 = h->kSlots - 2, s1 = h->kSlots - 1;
         mg_resid_inf<T>(h, L[0], s0);
         double r0[3] = {0, 0, 0};
@@ -964,10 +1007,19 @@ void stag_mg_solver(lmm_handle* h) {
 }
 
 // ------------------------------------------------------------ pressure V-cycle
+// zero: from phi = 0, whatever phi holds (its first launch writes it)
 template <class T>
-void cc_smooth(lmm_handle* h, LevelDev<T>& L, int nsweeps) {
+void cc_smooth(lmm_handle* h, LevelDev<T>& L, int nsweeps, bool zero = false) {
+    if (zero && nsweeps < 1) LMM_CK(cudaMemsetAsync(L.pphi, 0, L.n * sizeof(T), h->stream));
     for (int s = 0; s < nsweeps; ++s)
         for (int parity = 0; parity < 2; ++parity) {
+            if (zero && s == 0 && parity == 0) {
+                if (launch_cc_zero<T>(L, h->stream)) {
+                    check_launch();
+                    continue;
+                }
+                LMM_CK(cudaMemsetAsync(L.pphi, 0, L.n * sizeof(T), h->stream));
+            }
             launch_cc_smooth<T>(L, parity, h->stream, (h->knobs.smoother_order == 0 && parity == 1) ? 1 : 0);
             check_launch();
         }
@@ -981,20 +1033,21 @@ void macproject(lmm_handle* h) {
     const lmm_knobs& K = h->knobs;
     const int nl = h->nlev_p;
     const int lc = tail_start<T>(h, L, nl, false);
-    LMM_CK(cudaMemsetAsync(L[0].pphi, 0, L[0].n * sizeof(T), h->stream));
+    if (K.mg_max_vcycles < 1) LMM_CK(cudaMemsetAsync(L[0].pphi, 0, L[0].n * sizeof(T), h->stream));
     for (int vc = 0; vc < K.mg_max_vcycles; ++vc) {
-        for (int l = 1; l < std::min(lc, nl); ++l) LMM_CK(cudaMemsetAsync(L[l].pphi, 0, L[l].n * sizeof(T), h->stream));
+        // the first cycle starts from zero, as every coarse level does
+        auto from_zero = [&](int l) { return l > 0 || vc == 0; };
         for (int l = 0; l < lc && l < nl - 1; ++l) {
-            cc_smooth<T>(h, L[l], K.mg_nsmooths_down);
+            cc_smooth<T>(h, L[l], K.mg_nsmooths_down, from_zero(l));
             launch_cc_residual_restrict<T>(L[l], L[l + 1], h->stream);
             check_launch();
         }
         if (lc < nl) {
             LMM_CK(launch_ccmg_tail<T>(&L[lc], nl - lc, K.mg_nsmooths_down, K.mg_nsmooths_up, K.mg_nsmooths_bottom,
-                                       h->stream, lc > 0 || vc == 0));
+                                       h->stream, from_zero(lc)));
             check_launch();
         } else {
-            cc_smooth<T>(h, L[nl - 1], K.mg_nsmooths_bottom);
+            cc_smooth<T>(h, L[nl - 1], K.mg_nsmooths_bottom, from_zero(nl - 1));
         }
         for (int l = std::min(lc, nl - 1) - 1; l >= 0; --l) {
             launch_cc_prolong_add<T>(L[l], L[l + 1], h->stream);
@@ -1126,8 +1179,31 @@ void visc_schur(lmm_handle* h, T* mac, T* x_p) {
     }
 }
 
-// x = M^-1 b.  b_u / b_p and x_u / x_p are level-0 arrays of type T (they
-// may alias the level-0 rhs / phi arrays of the hierarchy).
+// sets pointers for a scope and puts the old ones back
+template <class T, int N>
+struct PtrSwap {
+    T** at[N];
+    T* old[N];
+    int n = 0;
+    void set(T*& p, T* v) {
+        at[n] = &p;
+        old[n++] = p;
+        p = v;
+    }
+    PtrSwap() = default;
+    ~PtrSwap() {
+        while (n > 0) {
+            --n;
+            *at[n] = old[n];
+        }
+    }
+    PtrSwap(const PtrSwap&) = delete;
+    PtrSwap& operator=(const PtrSwap&) = delete;
+};
+
+// x = M^-1 b.  b_u / b_p and x_u / x_p are level-0 arrays of type T, read
+// and written in place (x_u may not overlap b_u; both start on a pair of
+// entries).
 template <class T>
 void apply_precon(lmm_handle* h, const T* const b_u[3], const T* b_p, T* const x_u[3], T* x_p) {
     NvtxRange nvtx_("apply_precon");
@@ -1142,18 +1218,19 @@ void apply_precon(lmm_handle* h, const T* const b_u[3], const T* b_p, T* const x
     PrecScratch<T> S = prec_scratch<T>(h);
     const int mean_slot = h->batched ? lmm_handle::kBSlots - 1 : h->kSlots - 3;
 
-    // the staggered solve reads its rhs from L0.rhs and iterates on L0.phi
+    // the staggered solve works in place: its rhs is read where it is and
+    // x_u is the finest level's phi
     auto vel_solve = [&](const T* const rhs[3], bool zero_guess) {
+        PtrSwap<T, 6> swap;
         for (int d = 0; d < dm; ++d) {
-            if (rhs[d] != L0.rhs[d]) LMM_CK(cudaMemcpyAsync(L0.rhs[d], rhs[d], n * sizeof(T), cudaMemcpyDeviceToDevice, h->stream));
-            if (zero_guess) LMM_CK(cudaMemsetAsync(L0.phi[d], 0, n * sizeof(T), h->stream));
+            swap.set(L0.rhs[d], const_cast<T*>(rhs[d]));
+            swap.set(L0.phi[d], x_u[d]);
         }
-        stag_mg_solver<T>(h);
-        for (int d = 0; d < dm; ++d)
-            if (x_u[d] != L0.phi[d]) LMM_CK(cudaMemcpyAsync(x_u[d], L0.phi[d], n * sizeof(T), cudaMemcpyDeviceToDevice, h->stream));
+        stag_mg_solver<T>(h, zero_guess);
     };
     auto pres_solve = [&](const T* rhs) {
-        if (rhs != L0.prhs) LMM_CK(cudaMemcpyAsync(L0.prhs, rhs, n * sizeof(T), cudaMemcpyDeviceToDevice, h->stream));
+        PtrSwap<T, 1> swap;
+        swap.set(L0.prhs, const_cast<T*>(rhs));
         macproject<T>(h);
     };
     const T* xu_c[3] = {x_u[0], x_u[1], x_u[2]};
@@ -1183,10 +1260,7 @@ void apply_precon(lmm_handle* h, const T* const b_u[3], const T* b_p, T* const x
         vel_solve(b_u, true);
         launch_div_plus<T>(L0, xu_c, b_p, S.mac, h->stream);
         check_launch();
-        if (std::fabs(theta) > 0.0)
-            pres_solve(S.mac);
-        else
-            LMM_CK(cudaMemsetAsync(L0.pphi, 0, n * sizeof(T), h->stream));
+        if (std::fabs(theta) > 0.0) pres_solve(S.mac);  // (the Schur step reads no phi at theta = 0)
         if (K.visc_schur_approx == 1) {
             visc_schur<T>(h, S.mac, x_p);
             if (pt == -2 || pt == -5) {
@@ -1204,9 +1278,6 @@ void apply_precon(lmm_handle* h, const T* const b_u[3], const T* b_p, T* const x
             check_launch();
             const T* bt[3] = {S.butmp[0], S.butmp[1], S.butmp[2]};
             // second viscous solve starts from the current x_u (apply_precon.f90:276)
-            for (int d = 0; d < dm; ++d)
-                if (x_u[d] != L0.phi[d])
-                    LMM_CK(cudaMemcpyAsync(L0.phi[d], x_u[d], n * sizeof(T), cudaMemcpyDeviceToDevice, h->stream));
             vel_solve(bt, false);
         }
         break;
@@ -1217,10 +1288,7 @@ void apply_precon(lmm_handle* h, const T* const b_u[3], const T* b_p, T* const x
             launch_scale_copy<T>(S.mac, S.mac, -1.0, n, h->stream);
             check_launch();
         }
-        if (std::fabs(theta) > 0.0)
-            pres_solve(S.mac);
-        else
-            LMM_CK(cudaMemsetAsync(L0.pphi, 0, n * sizeof(T), h->stream));
+        if (std::fabs(theta) > 0.0) pres_solve(S.mac);  // (the Schur step reads no phi at theta = 0)
         if (K.visc_schur_approx == 1) {
             visc_schur<T>(h, S.mac, x_p);
         } else {
@@ -1264,7 +1332,7 @@ void apply_precon(lmm_handle* h, const T* const b_u[3], const T* b_p, T* const x
 }
 
 // Run `body` (a fixed sequence of launches on h->stream) through a CUDA graph
-// keyed by (in, out, theta, precision): the first call runs eagerly (kernel
+// keyed by (in, out, theta, precision, uniform coefficients): the first call runs eagerly (kernel
 // attributes get set), the second captures and instantiates, later calls
 // replay.  Launch and V-cycle counters advance as if launched eagerly.
 template <class F>
@@ -1274,7 +1342,7 @@ void run_graphed(lmm_handle* h, const void* in, const void* out, int prec, F bod
         body();
         return;
     }
-    auto key = std::make_tuple(in, out, h->theta_loaded, prec);
+    auto key = std::make_tuple(in, out, h->theta_loaded, prec, h->uniform_id);
     lmm_handle::Graph& g = h->graphs[key];
     if (g.exec) {
         LMM_CK(cudaGraphLaunch(g.exec, h->stream));
@@ -2513,8 +2581,7 @@ int lmm_stokes_update_knobs(lmm_handle* h, const lmm_knobs* k) {
 int lmm_stokes_destroy(lmm_handle* h) {
     if (!h) return LMM_OK;
     if (h->stream) cudaStreamSynchronize(h->stream);
-    for (auto& kv : h->graphs)
-        if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+    h->drop_graphs();
     bc_remove(h->arena);
     bc_remove(h->lrn_block);
     if (h->arena) cudaFree(h->arena);

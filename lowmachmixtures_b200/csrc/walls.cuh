@@ -69,6 +69,17 @@ void wl_gs_colour(const LevelDev<T>& L, int visc, int color, const T* const rhs[
 }
 
 template <class T>
+void wl_gs_zero(const LevelDev<T>& L, int visc, const T* const rhs[3], T* const phi[3], double omega, cudaStream_t s) {
+    const T dxsqinv = T(1.0 / (L.dx * L.dx)), om = (T)omega;
+    const G3 g = geom3(L.D.nx / 2, L.D.ny, L.D.nz);
+    if (L.D.dm == 2) {
+        LMM_VISC_DISPATCH(visc, launch_pdl(k_gs_zero<T, 2, V, true>, g.grid, g.block, 0, s, L.D, L.coef(), rhs[0], phi[0], phi[1], phi[1], om, dxsqinv))
+    } else {
+        LMM_VISC_DISPATCH(visc, launch_pdl(k_gs_zero<T, 3, V, true>, g.grid, g.block, 0, s, L.D, L.coef(), rhs[0], phi[0], phi[1], phi[2], om, dxsqinv))
+    }
+}
+
+template <class T>
 void wl_jacobi(const LevelDev<T>& L, int visc, const T* const rhs[3], const T* const pin[3], T* const pout[3], double omega,
                cudaStream_t s) {
     const T dxsqinv = T(1.0 / (L.dx * L.dx));
@@ -109,6 +120,7 @@ void wl_prolong_add(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const 
 }
 
 #define LMM_INSTANTIATE_WALLS(T)                                                                                           \
+    template void wl_gs_zero<T>(const LevelDev<T>&, int, const T* const[3], T* const[3], double, cudaStream_t); \
     template void wl_applyop<T>(const LevelDev<T>&, int, const T* const[3], T* const[3], cudaStream_t, int);              \
     template void wl_gs_colour<T>(const LevelDev<T>&, int, int, const T* const[3], T* const[3], double, cudaStream_t, int); \
     template void wl_jacobi<T>(const LevelDev<T>&, int, const T* const[3], const T* const[3], T* const[3], double,         \
