@@ -74,8 +74,7 @@ __global__ void __launch_bounds__(kT, (VISC == 3 || VISC == -3) ? 3 : 4) k_apply
 }
 
 template <class TX>
-static void apply_matrix_impl(const LevelDev<double>& L0, int visc, const TX* xb, int64_t n, int dm, const SVec& b,
-                              cudaStream_t s) {
+static void apply_matrix_impl(const LevelDev<double>& L0, int visc, const TX* const x[4], double* const b[4], cudaStream_t s) {
     const double dxsqinv = 1.0 / (L0.dx * L0.dx);
     const double dxinv = 1.0 / L0.dx;
     // periodic grids: the block shape the autotuner chose (a shape it
@@ -90,16 +89,13 @@ static void apply_matrix_impl(const LevelDev<double>& L0, int visc, const TX* xb
     }
     if (by > L0.D.ny) by = L0.D.ny;
     const dim3 blk(bx, by, 1), grd((L0.D.nx + bx - 1) / bx, (L0.D.ny + by - 1) / by, L0.D.nz);
-    const TX* x0 = xb;
-    const TX* x1 = xb + n;
-    const TX* x2 = (dm == 3) ? xb + 2 * n : xb;
-    const TX* xp = xb + (int64_t)dm * n;
-    double* b2 = (b.dm == 3) ? b.c(2) : b.c(0);
+    const TX *x0 = x[0], *x1 = x[1], *x2 = x[2], *xp = x[3];
+    const int dm = L0.D.dm;
 #define AM(DM_, V_)                                                                                                        \
     if (L0.D.wall)                                                                                                         \
-        launch_pdl(k_apply_matrix<DM_, V_, TX, true>, grd, blk, 0, s, L0.D, L0.coef(), x0, x1, x2, xp, b.c(0), b.c(1), b2, b.p(), dxsqinv, dxinv); \
+        launch_pdl(k_apply_matrix<DM_, V_, TX, true>, grd, blk, 0, s, L0.D, L0.coef(), x0, x1, x2, xp, b[0], b[1], b[2], b[3], dxsqinv, dxinv); \
     else                                                                                                                   \
-        launch_pdl(k_apply_matrix<DM_, V_, TX>, grd, blk, 0, s, L0.D, L0.coef(), x0, x1, x2, xp, b.c(0), b.c(1), b2, b.p(), dxsqinv, dxinv)
+        launch_pdl(k_apply_matrix<DM_, V_, TX>, grd, blk, 0, s, L0.D, L0.coef(), x0, x1, x2, xp, b[0], b[1], b[2], b[3], dxsqinv, dxinv)
 #define AMV(DM_)                    \
     switch (visc) {                 \
     case -1: AM(DM_, -1); break;    \
@@ -118,12 +114,20 @@ static void apply_matrix_impl(const LevelDev<double>& L0, int visc, const TX* xb
 #undef AM
 }
 
+// (2D: the third face arrays are not touched)
+void launch_apply_matrix(const LevelDev<double>& L0, int visc, const double* const x[4], double* const b[4], cudaStream_t s) {
+    apply_matrix_impl<double>(L0, visc, x, b, s);
+}
 void launch_apply_matrix(const LevelDev<double>& L0, int visc, const SVec& x, const SVec& b, cudaStream_t s) {
-    apply_matrix_impl<double>(L0, visc, x.base, x.n, x.dm, b, s);
+    const double* xs[4] = {x.c(0), x.c(1), x.dm == 3 ? x.c(2) : x.c(0), x.p()};
+    double* bs[4] = {b.c(0), b.c(1), b.dm == 3 ? b.c(2) : b.c(0), b.p()};
+    apply_matrix_impl<double>(L0, visc, xs, bs, s);
 }
 void launch_apply_matrix_f32(const LevelDev<double>& L0, int visc, const float* x, int64_t n, int dm, const SVec& b,
                              cudaStream_t s) {
-    apply_matrix_impl<float>(L0, visc, x, n, dm, b, s);
+    const float* xs[4] = {x, x + n, dm == 3 ? x + 2 * n : x, x + (int64_t)dm * n};
+    double* bs[4] = {b.c(0), b.c(1), b.dm == 3 ? b.c(2) : b.c(0), b.p()};
+    apply_matrix_impl<float>(L0, visc, xs, bs, s);
 }
 
 __global__ void k_neg_resid(double* __restrict__ out, const double* __restrict__ b, int64_t n) {

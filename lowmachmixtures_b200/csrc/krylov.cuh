@@ -61,6 +61,8 @@ void launch_add_scaled_multi_f32(double* x, const MZ32& Z, const YS& ys, int J, 
 void launch_div_by_f32(const double* w, double* v, float* v32, const double* den, int64_t n, cudaStream_t s);
 
 void launch_apply_matrix(const LevelDev<double>& L0, int visc, const SVec& x, const SVec& b, cudaStream_t s);
+// on separate arrays {u_x, u_y, u_z, p}: x is read through the read-only path, so no array of b may overlap it
+void launch_apply_matrix(const LevelDev<double>& L0, int visc, const double* const x[4], double* const b[4], cudaStream_t s);
 // the same operator applied to an FP32 Stokes vector (FGMRES Z storage), FP64 arithmetic
 void launch_apply_matrix_f32(const LevelDev<double>& L0, int visc, const float* x, int64_t n, int dm, const SVec& b,
                              cudaStream_t s);

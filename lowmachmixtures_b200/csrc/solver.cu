@@ -3026,6 +3026,31 @@ extern "C" int lmm_op_apply_matrix(lmm_handle* h, const double* const x_u[3], co
     try {
         const int dm = h->dm;
         const int64_t n = h->n;
+        // the caller's arrays in place, unless an output overlaps an input or
+        // another output (then through the handle's vectors)
+        {
+            const double* x[4] = {x_u[0], x_u[1], dm == 3 ? x_u[2] : x_u[0], x_p};
+            double* b[4] = {b_u[0], b_u[1], dm == 3 ? b_u[2] : b_u[0], b_p};
+            auto apart = [&](const double* p, const double* q) {
+                const uintptr_t a = (uintptr_t)p, c = (uintptr_t)q, len = (uintptr_t)n * sizeof(double);
+                return a + len <= c || c + len <= a;
+            };
+            bool ok = true;
+            for (int i = 0; i < 4; ++i) {
+                if (dm == 2 && i == 2) continue;
+                for (int j = 0; j < 4; ++j) {
+                    if (dm == 2 && j == 2) continue;
+                    ok = ok && apart(b[i], x[j]) && (i == j || apart(b[i], b[j]));
+                }
+            }
+            if (ok) {
+                lmm::BcScope scope({x[0], x[1], x[2], x[3], b[0], b[1], b[2], b[3]}, (size_t)n * sizeof(double));
+                launch_apply_matrix(h->L64[0], h->knobs.visc_type, x, b, h->stream);
+                check_launch();
+                LMM_CK(host_wait(h));
+                return bc_status();
+            }
+        }
         for (int d = 0; d < dm; ++d)
             LMM_CK(cudaMemcpyAsync(h->r.c(d), x_u[d], n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
         LMM_CK(cudaMemcpyAsync(h->r.p(), x_p, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
