@@ -37,6 +37,7 @@ UNITS = [
     ("walls_fp32.cu", ["-fmad=true"]),
     ("krylov.cu", ["-fmad=false"]),
     ("solver.cu", ["-fmad=false"]),
+    ("coeffs.cu", ["-fmad=false"]),
     ("noalloc.cu", ["-fmad=false"]),
     ("autotune.cu", []),
     ("nn.cu", ["-fmad=true"]),

@@ -644,75 +644,21 @@ __device__ __forceinline__ T fat(const T* a, const Dims& F, int i, int j, int k)
     return ld(a, i + F.nx * (j + F.ny * k));
 }
 
-// do_visc: 0 faces only, 1 faces + cells + edges, 2 faces + cells (the edges
-// of a grid with walls go through k_coarsen_edges_w)
+// face coefficients of a coarse level: the mean of the fine faces each covers
 template <class T, int DM>
-__global__ void __launch_bounds__(kThreads) k_coarsen(Dims F, Dims Dc, Coef<T> Cf, T* a0, T* a1, T* a2, T* beta, T* gamma,
-                                                      T* e0, T* e1, T* e2, int do_visc) {
+__global__ void __launch_bounds__(kThreads) k_coarsen_faces(Dims F, Dims Dc, const T* A0, const T* A1, const T* A2, T* a0, T* a1, T* a2) {
     const Pos q = pos3(Dc.nx, Dc.ny);
     if (!q.ok) return;
     const int i = q.i, j = q.j, k = q.k;
     const int t = i + Dc.nx * (j + Dc.ny * k);
     const int I = 2 * i, J = 2 * j, K = 2 * k;
     if constexpr (DM == 2) {
-        a0[t] = T(0.5) * (fat(Cf.alpha[0], F, I, J, k) + fat(Cf.alpha[0], F, I, J + 1, k));
-        a1[t] = T(0.5) * (fat(Cf.alpha[1], F, I, J, k) + fat(Cf.alpha[1], F, I + 1, J, k));
-        if (do_visc) {
-            const T* b = Cf.beta;
-            beta[t] = T(0.25) * (fat(b, F, I, J, k) + fat(b, F, I + 1, J, k) + fat(b, F, I, J + 1, k) + fat(b, F, I + 1, J + 1, k));
-            const T* g = Cf.gamma;
-            gamma[t] = T(0.25) * (fat(g, F, I, J, k) + fat(g, F, I + 1, J, k) + fat(g, F, I, J + 1, k) + fat(g, F, I + 1, J + 1, k));
-            if (do_visc == 1) e0[t] = fat(Cf.bed[0], F, I, J, k);  // nodal injection
-        }
+        a0[t] = T(0.5) * (fat(A0, F, I, J, k) + fat(A0, F, I, J + 1, k));
+        a1[t] = T(0.5) * (fat(A1, F, I, J, k) + fat(A1, F, I + 1, J, k));
     } else {
-        const T* A0 = Cf.alpha[0];
-        const T* A1 = Cf.alpha[1];
-        const T* A2 = Cf.alpha[2];
         a0[t] = T(0.25) * (fat(A0, F, I, J, K) + fat(A0, F, I, J + 1, K) + fat(A0, F, I, J, K + 1) + fat(A0, F, I, J + 1, K + 1));
         a1[t] = T(0.25) * (fat(A1, F, I, J, K) + fat(A1, F, I + 1, J, K) + fat(A1, F, I, J, K + 1) + fat(A1, F, I + 1, J, K + 1));
         a2[t] = T(0.25) * (fat(A2, F, I, J, K) + fat(A2, F, I + 1, J, K) + fat(A2, F, I, J + 1, K) + fat(A2, F, I + 1, J + 1, K));
-        if (do_visc) {
-            const T* b = Cf.beta;
-            beta[t] = T(0.125) * (fat(b, F, I, J, K) + fat(b, F, I + 1, J, K) + fat(b, F, I, J + 1, K) + fat(b, F, I + 1, J + 1, K) +
-                                  fat(b, F, I, J, K + 1) + fat(b, F, I + 1, J, K + 1) + fat(b, F, I, J + 1, K + 1) +
-                                  fat(b, F, I + 1, J + 1, K + 1));
-            const T* g = Cf.gamma;
-            gamma[t] = T(0.125) * (fat(g, F, I, J, K) + fat(g, F, I + 1, J, K) + fat(g, F, I, J + 1, K) + fat(g, F, I + 1, J + 1, K) +
-                                   fat(g, F, I, J, K + 1) + fat(g, F, I + 1, J, K + 1) + fat(g, F, I, J + 1, K + 1) +
-                                   fat(g, F, I + 1, J + 1, K + 1));
-            if (do_visc == 1) {
-                e0[t] = T(0.5) * (fat(Cf.bed[0], F, I, J, K) + fat(Cf.bed[0], F, I, J, K + 1));
-                e1[t] = T(0.5) * (fat(Cf.bed[1], F, I, J, K) + fat(Cf.bed[1], F, I, J + 1, K));
-                e2[t] = T(0.5) * (fat(Cf.bed[2], F, I, J, K) + fat(Cf.bed[2], F, I + 1, J, K));
-            }
-        }
-    }
-}
-
-// edge coefficients of a grid with walls (n+1 nodes along a nodal
-// wall-bounded direction): nodal injection in 2D (nodal_restriction,
-// stag_mg_solver.f90:1229-1244), two-point average along the edge in 3D
-// (edge_restriction, :1326-1367); the launch covers (nx+1, ny+1, nz+1)
-template <class T, int DM>
-__global__ void __launch_bounds__(kThreads) k_coarsen_edges_w(Dims F, Dims Dc, const T* f0, const T* f1, const T* f2, T* e0, T* e1,
-                                                              T* e2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    const int I = 2 * i, J = 2 * j, K = 2 * k;
-    const T* f[3] = {f0, f1, f2};
-    T* e[3] = {e0, e1, e2};
-#pragma unroll
-    for (int q = 0; q < (DM == 2 ? 1 : 3); ++q) {
-        // 2D: the third index is the instance (a batch stacks nz of them)
-        const int cx = edge_ext(Dc, q, 0), cy = edge_ext(Dc, q, 1), cz = (DM == 3) ? edge_ext(Dc, q, 2) : Dc.nz;
-        if (i >= cx || j >= cy || k >= cz) continue;
-        const int fx = edge_ext(F, q, 0), fy = edge_ext(F, q, 1);
-        auto at = [&](int a, int b, int c) { return ld(f[q], a + fx * (b + fy * c)); };
-        T v;
-        if (DM == 2) v = at(I, J, k);
-        else if (q == 0) v = T(0.5) * (at(I, J, K) + at(I, J, K + 1));
-        else if (q == 1) v = T(0.5) * (at(I, J, K) + at(I, J + 1, K));
-        else v = T(0.5) * (at(I, J, K) + at(I + 1, J, K));
-        e[q][i + cx * (j + cy * k)] = v;
     }
 }
 
@@ -765,24 +711,6 @@ __device__ __forceinline__ T cc_update(const T* const a[3], T c, const T* phi, c
     const T p = ldp<LD>(phi, n.s);
     const T res = ldp<LD>(rhs, n.s) - cc_lap_vals<T, DM>(k, p, nb, dxsqinv);
     return p + res / cc_diag_vals<T, DM>(k, dxsqinv);
-}
-
-// flag = 1 when an entry of a0, a1 or a2 (a1, a2 may be null) differs from
-// a0[0] in its bits
-template <class T>
-__global__ void k_uniform_check(const T* __restrict__ a0, const T* __restrict__ a1, const T* __restrict__ a2, int64_t n,
-                                int* __restrict__ flag) {
-    auto bits = [](T x) -> unsigned long long {
-        if constexpr (sizeof(T) == 8)
-            return (unsigned long long)__double_as_longlong((double)x);
-        else
-            return (unsigned long long)(unsigned)__float_as_int((float)x);
-    };
-    const unsigned long long v = bits(a0[0]);
-    bool diff = false;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n && !diff; t += (int64_t)gridDim.x * blockDim.x)
-        diff = bits(a0[t]) != v || (a1 && bits(a1[t]) != v) || (a2 && bits(a2[t]) != v);
-    if (diff) atomicOr(flag, 1);
 }
 
 // U: every face coefficient equals cu (the arrays a0..a2 are not read);
@@ -954,19 +882,6 @@ __global__ void k_add_to(T* __restrict__ x, const T* __restrict__ y, int64_t n) 
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t < n) x[t] = x[t] + y[t];
 }
-template <class T>
-__global__ void k_recip(const T* __restrict__ in, T* __restrict__ out, int64_t n) {
-    pdl_enter();
-    int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t < n) out[t] = T(1) / in[t];
-}
-template <class T>
-__global__ void k_fill(T* __restrict__ out, T v, int64_t n) {
-    pdl_enter();
-    int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t < n) out[t] = v;
-}
-
 // --------------------------------------------------------------- deterministic reductions
 // Each block accumulates a fixed grid-stride subset in double, reduces it in
 // a fixed tree, writes its partials; the last block to finish sums all
@@ -1429,31 +1344,12 @@ void launch_prolong_add(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* co
 }
 
 template <class T>
-void launch_coarsen_coeffs(const LevelDev<T>& F, const LevelDev<T>& Cc, bool pressure_faces, cudaStream_t s) {
+void launch_coarsen_faces(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const f[3], T* const c[3], cudaStream_t s) {
     const G3 g = geom3(Cc.D.nx, Cc.D.ny, Cc.D.nz);
-    Coef<T> cf = F.coef();
-    cf.alpha_uniform = 0;  // the arrays are read (and may be others below)
-    if (pressure_faces) {
-        for (int d = 0; d < 3; ++d) cf.alpha[d] = F.pa[d];
-        if (F.D.dm == 2)
-            k_coarsen<T, 2><<<g.grid, g.block, 0, s>>>(F.D, Cc.D, cf, Cc.pa[0], Cc.pa[1], Cc.pa[2], nullptr, nullptr, nullptr, nullptr, nullptr, 0);
-        else
-            k_coarsen<T, 3><<<g.grid, g.block, 0, s>>>(F.D, Cc.D, cf, Cc.pa[0], Cc.pa[1], Cc.pa[2], nullptr, nullptr, nullptr, nullptr, nullptr, 0);
-        return;
-    }
-    const int dv = F.D.wall ? 2 : 1;
     if (F.D.dm == 2)
-        k_coarsen<T, 2><<<g.grid, g.block, 0, s>>>(F.D, Cc.D, cf, Cc.alpha[0], Cc.alpha[1], Cc.alpha[2], Cc.beta, Cc.gamma, Cc.bed[0], Cc.bed[1], Cc.bed[2], dv);
+        k_coarsen_faces<T, 2><<<g.grid, g.block, 0, s>>>(F.D, Cc.D, f[0], f[1], nullptr, c[0], c[1], nullptr);
     else
-        k_coarsen<T, 3><<<g.grid, g.block, 0, s>>>(F.D, Cc.D, cf, Cc.alpha[0], Cc.alpha[1], Cc.alpha[2], Cc.beta, Cc.gamma, Cc.bed[0], Cc.bed[1], Cc.bed[2], dv);
-    if (F.D.wall) {
-        count_launch();
-        const G3 ge = geom3(Cc.D.nx + 1, Cc.D.ny + 1, Cc.D.dm == 3 ? Cc.D.nz + 1 : Cc.D.nz);
-        if (F.D.dm == 2)
-            k_coarsen_edges_w<T, 2><<<ge.grid, ge.block, 0, s>>>(F.D, Cc.D, F.bed[0], F.bed[1], F.bed[2], Cc.bed[0], Cc.bed[1], Cc.bed[2]);
-        else
-            k_coarsen_edges_w<T, 3><<<ge.grid, ge.block, 0, s>>>(F.D, Cc.D, F.bed[0], F.bed[1], F.bed[2], Cc.bed[0], Cc.bed[1], Cc.bed[2]);
-    }
+        k_coarsen_faces<T, 3><<<g.grid, g.block, 0, s>>>(F.D, Cc.D, f[0], f[1], f[2], c[0], c[1], c[2]);
 }
 
 template <class T>
@@ -1497,14 +1393,6 @@ bool launch_cc_zero(const LevelDev<T>& L, cudaStream_t s) {
     }
 #undef CZ
     return true;
-}
-
-template <class T>
-void launch_uniform_check(const LevelDev<T>& L, int* flag, cudaStream_t s, bool velocity) {
-    const int64_t n = L.n;
-    const int blocks = (int)std::min<int64_t>((n + kThreads - 1) / kThreads, 1184);
-    T* const* a = velocity ? L.alpha : L.pa;
-    k_uniform_check<T><<<blocks, kThreads, 0, s>>>(a[0], a[1], L.D.dm == 3 ? a[2] : nullptr, n, flag);
 }
 
 template <class T>
@@ -1594,15 +1482,6 @@ void launch_scale_copy(const T* in, T* out, double scale, int64_t n, cudaStream_
     launch_pdl(k_scale_copy<T>, nblocks_for(n), kThreads, 0, s, in, out, (T)scale, n);
 }
 template <class T>
-void launch_recip(const T* in, T* out, int64_t n, cudaStream_t s) {
-    launch_pdl(k_recip<T>, nblocks_for(n), kThreads, 0, s, in, out, n);
-}
-template <class T>
-void launch_fill(T* out, double v, int64_t n, cudaStream_t s) {
-    launch_pdl(k_fill<T>, nblocks_for(n), kThreads, 0, s, out, (T)v, n);
-}
-
-template <class T>
 void launch_reduce(const Dims& D, int mode, const T* const a[4], const T* const b[4], const double wseam[3], double pw,
                    double* partials, unsigned* counter, double* out, int nblocks, cudaStream_t s, int ninst) {
     const dim3 grid(nblocks, ninst);
@@ -1670,18 +1549,15 @@ namespace lmm {
     template void launch_residual_restrict<T>(const LevelDev<T>&, const LevelDev<T>&, int, const T* const[3],                  \
                                               const T* const[3], T* const[3], cudaStream_t, int);                              \
     template void launch_prolong_add<T>(const LevelDev<T>&, const LevelDev<T>&, const T* const[3], T* const[3], cudaStream_t); \
-    template void launch_coarsen_coeffs<T>(const LevelDev<T>&, const LevelDev<T>&, bool, cudaStream_t);                        \
+    template void launch_coarsen_faces<T>(const LevelDev<T>&, const LevelDev<T>&, const T* const[3], T* const[3], cudaStream_t); \
     template void launch_cc_smooth<T>(const LevelDev<T>&, int, cudaStream_t, int);                                              \
     template void launch_cc_residual_restrict<T>(const LevelDev<T>&, const LevelDev<T>&, cudaStream_t);                        \
     template void launch_cc_prolong_add<T>(const LevelDev<T>&, const LevelDev<T>&, cudaStream_t);                              \
-    template void launch_uniform_check<T>(const LevelDev<T>&, int*, cudaStream_t, bool);                                            \
     template void launch_neg_cc_lap<T>(const LevelDev<T>&, const T*, T*, cudaStream_t);                                        \
     template void launch_div_plus<T>(const LevelDev<T>&, const T* const[3], const T*, T*, cudaStream_t);                        \
     template void launch_sub_weighted_grad<T>(const LevelDev<T>&, const T* const[3], const T*, T* const[3], cudaStream_t);     \
     template void launch_scale_copy<T>(const T*, T*, double, int64_t, cudaStream_t);                                           \
     template void launch_add_to<T>(T*, const T*, int64_t, cudaStream_t);                                                      \
-    template void launch_recip<T>(const T*, T*, int64_t, cudaStream_t);                                                        \
-    template void launch_fill<T>(T*, double, int64_t, cudaStream_t);                                                           \
     template void launch_reduce<T>(const Dims&, int, const T* const[4], const T* const[4], const double[3], double,            \
                                    double*, unsigned*, double*, int, cudaStream_t, int);                                      \
     template bool gs_tma_supported<T>(const LevelDev<T>&, int, int, int);                                                     \

@@ -99,8 +99,9 @@ void launch_residual_restrict(const LevelDev<T>& F, const LevelDev<T>& Cc, int v
 template <class T>
 void launch_prolong_add(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const phi_c[3], T* const phi_f[3],
                         cudaStream_t s);
+// c = the coarse faces' means of the fine face coefficients f
 template <class T>
-void launch_coarsen_coeffs(const LevelDev<T>& F, const LevelDev<T>& Cc, bool pressure_faces, cudaStream_t s);
+void launch_coarsen_faces(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const f[3], T* const c[3], cudaStream_t s);
 
 // The same four operations on a grid with walls (walls.cuh; the launchers
 // above hand wall-bounded levels to these)
@@ -141,10 +142,6 @@ template <class T>
 bool launch_cc_zero(const LevelDev<T>& L, cudaStream_t s);
 template <class T>
 void launch_cc_residual_restrict(const LevelDev<T>& F, const LevelDev<T>& Cc, cudaStream_t s);
-// *flag |= 1 when the level's pressure face coefficients are not all the
-// same value (bit for bit)
-template <class T>
-void launch_uniform_check(const LevelDev<T>& L, int* flag, cudaStream_t s, bool velocity = false);
 template <class T>
 void launch_cc_prolong_add(const LevelDev<T>& F, const LevelDev<T>& Cc, cudaStream_t s);
 template <class T>
@@ -177,10 +174,6 @@ void launch_scale_copy(const T* in, T* out, double scale, int64_t n, cudaStream_
 // x = x + y
 template <class T>
 void launch_add_to(T* x, const T* y, int64_t n, cudaStream_t s);
-template <class T>
-void launch_recip(const T* in, T* out, int64_t n, cudaStream_t s);
-template <class T>
-void launch_fill(T* out, double v, int64_t n, cudaStream_t s);
 
 // Deterministic weighted sums over one level-0 vector:
 //   mode 0: out[c] = sum_w a_c * b_c   (stag_inner_prod / cc_inner_prod weights)

@@ -32,6 +32,7 @@
 #include "../../include/lmm_ensemble.h"
 #include "../../include/lmm_noalloc.h"
 #include "../../include/lmm_stokes.h"
+#include "coeffs.cuh"
 #include "kernels.h"
 #include "krylov.cuh"
 #include "learned.cuh"
@@ -264,7 +265,8 @@ struct lmm_handle {
     unsigned* counter = nullptr;
     double* scal = nullptr;       // device scalar slots (8 doubles per slot)
     double* hscal = nullptr;      // pinned host mirror
-    double* hmisc = nullptr;      // pinned: per-level pressure coefficients and flags (64 doubles)
+    double* hmisc = nullptr;      // pinned mirror of ustate (64 doubles)
+    double* ustate = nullptr;     // uniform coefficients: 32 values, 32 flags, one unread value and flag (64 doubles)
     int red_blocks = 0;
     static constexpr int kSlots = 256;
     // BoxLib staging
@@ -275,6 +277,7 @@ struct lmm_handle {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t wait_ev = nullptr;  // knobs.host_wait = 1: host waits block instead of spinning
     cudaEvent_t col_ev = nullptr;   // FGMRES: the Hessenberg column has reached the host
+    double norm_b = 0.0;            // |b| of the current solve
     bool coeffs_loaded = false;
     double theta_loaded = 0.0;
     // captured preconditioner applications: (input, output, theta, precision, uniform_id)
@@ -442,6 +445,7 @@ size_t plan_bytes(const lmm_grid& g, const lmm_knobs& k, int nlev, int nlev_p, i
     add(partials_count(g, batch), sizeof(double));  // reduction partials
     add(std::max(64, batch), sizeof(unsigned));
     add(64, sizeof(int));  // error word of the kernels with bounded waits
+    add(64, sizeof(double));  // uniform-coefficient values and flags
     add(8 * lmm_handle::kSlots, sizeof(double));
     // BoxLib staging: the largest field with up to 4 ghost layers
     int64_t st = 1;
@@ -496,7 +500,9 @@ void build_levels(lmm_handle* h) {
             }
         }
         if (l < h->nlev_p) {
-            for (int d = 0; d < dm; ++d) v.pa[d] = h->alloc<T>(v.n);
+            // the finest level of a periodic box shares 1/alpha (create_impl)
+            if (l > 0 || h->D0.wall)
+                for (int d = 0; d < dm; ++d) v.pa[d] = h->alloc<T>(v.n);
             if (h->knobs.visc_schur_approx == 1)
                 for (int d = 0; d < dm; ++d) v.pmu[d] = h->alloc<T>(v.n);
             v.pphi = h->alloc<T>(v.n);
@@ -593,98 +599,111 @@ double read_slot(lmm_handle* h, int slot, int idx) {
 // V-cycle), 1/alpha for the pressure solve and the FP32 copies.
 void load_coeffs(lmm_handle* h, const double* const alpha_dev[3], const double* beta, const double* const bed[3],
                  const double* gamma, double theta) {
-    const int dm = h->dm;
+    const int dm = h->dm, nedge = dm == 2 ? 1 : 3;
+    const bool fp32 = h->knobs.precision == LMM_PRECISION_FP32;
     LevelDev<double>& L0 = h->L64[0];
-    const int64_t n = h->n;
-    for (int d = 0; d < dm; ++d) {
-        if (alpha_dev[d] != h->alpha_fc[d])
-            LMM_CK(cudaMemcpyAsync(h->alpha_fc[d], alpha_dev[d], n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-        launch_scale_copy<double>(h->alpha_fc[d], L0.alpha[d], theta, n, h->stream);
-        launch_recip<double>(h->alpha_fc[d], h->alphainv[d], n, h->stream);
+    // flags and values of the uniform levels (see below): 32 values, 32 flags
+    double* vals = h->ustate;
+    int* flags = reinterpret_cast<int*>(h->ustate + 32);
+    double* dump_v = h->ustate + 48;   // of levels past the 16 that are kept
+    int* dump_f = reinterpret_cast<int*>(h->ustate + 49);
+    LMM_CK(cudaMemsetAsync(flags, 0, 32 * sizeof(int), h->stream));
+    auto slots = [&](int l, double*& va, double*& vp, int*& fa, int*& fp) {
+        va = l < 16 ? vals + 16 + l : dump_v;
+        vp = l < 16 ? vals + l : dump_v;
+        fa = l < 16 ? flags + 16 + l : dump_f;
+        fp = l < 16 ? flags + l : dump_f;
+    };
+    {
+        CoefFine A{};
+        A.D = L0.D;
+        A.theta = theta;
+        A.beta = beta;
+        A.gamma = gamma;
+        A.o_beta = L0.beta;
+        A.o_gamma = L0.gamma;
+        for (int d = 0; d < dm; ++d) {
+            A.alpha[d] = alpha_dev[d];
+            A.o_alpha[d] = L0.alpha[d];
+            A.o_ainv[d] = h->alphainv[d];
+            if (h->D0.wall && h->nlev_p > 0) A.o_pa[d] = L0.pa[d];
+        }
+        for (int e = 0; e < nedge; ++e) {
+            A.bed[e] = bed[e];
+            A.ne[e] = edge_count(L0.D, e);
+            A.o_bed[e] = L0.bed[e];
+        }
+        if (fp32) {
+            LevelDev<float>& f = h->L32[0];
+            A.f_beta = f.beta;
+            A.f_gamma = f.gamma;
+            for (int d = 0; d < dm; ++d) {
+                A.f_alpha[d] = f.alpha[d];
+                A.f_ainv[d] = h->alphainv32[d];
+                A.f_pa[d] = f.pa[d];
+            }
+            for (int e = 0; e < nedge; ++e) A.f_bed[e] = f.bed[e];
+        }
+        slots(0, A.val_a, A.val_p, A.flag_a, A.flag_p);
+        launch_coeffs_fine(A, h->stream);
         check_launch();
     }
-    if (beta != L0.beta) LMM_CK(cudaMemcpyAsync(L0.beta, beta, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    if (gamma) {
-        if (gamma != L0.gamma) LMM_CK(cudaMemcpyAsync(L0.gamma, gamma, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    } else {
-        LMM_CK(cudaMemsetAsync(L0.gamma, 0, n * sizeof(double), h->stream));
-    }
-    for (int e = 0; e < (dm == 2 ? 1 : 3); ++e)
-        if (bed[e] != L0.bed[e])
-            LMM_CK(cudaMemcpyAsync(L0.bed[e], bed[e], edge_count(L0.D, e) * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    for (int l = 1; l < h->nlev; ++l) {
-        launch_coarsen_coeffs<double>(h->L64[l - 1], h->L64[l], false, h->stream);
+    for (int l = 1; l < (int)h->L64.size(); ++l) {
+        const LevelDev<double>&F = h->L64[l - 1], &C = h->L64[l];
+        CoefCoarse A{};
+        A.F = F.D;
+        A.C = C.D;
+        const bool hv = l < h->nlev, hp = l < h->nlev_p;
+        A.beta = F.beta;
+        A.gamma = F.gamma;
+        A.o_beta = C.beta;
+        A.o_gamma = C.gamma;
+        for (int d = 0; d < dm; ++d) {
+            if (hv) A.alpha[d] = F.alpha[d];
+            if (hp) A.pa[d] = F.pa[d];
+            A.o_alpha[d] = C.alpha[d];
+            A.o_pa[d] = C.pa[d];
+        }
+        for (int e = 0; e < nedge; ++e) {
+            A.bed[e] = F.bed[e];
+            A.o_bed[e] = C.bed[e];
+        }
+        if (fp32) {
+            const LevelDev<float>& f = h->L32[l];
+            A.f_beta = f.beta;
+            A.f_gamma = f.gamma;
+            for (int d = 0; d < dm; ++d) {
+                A.f_alpha[d] = f.alpha[d];
+                A.f_pa[d] = f.pa[d];
+            }
+            for (int e = 0; e < nedge; ++e) A.f_bed[e] = f.bed[e];
+        }
+        slots(l, A.val_a, A.val_p, A.flag_a, A.flag_p);
+        launch_coeffs_coarse(A, h->stream);
         check_launch();
-    }
-    // pressure face coefficients 1/alpha_fc, coarsened by face averaging
-    if (h->nlev_p > 0) {
-        for (int d = 0; d < dm; ++d)
-            LMM_CK(cudaMemcpyAsync(h->L64[0].pa[d], h->alphainv[d], n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-        if (h->D0.wall) {
-            // homogeneous Neumann pressure at walls: no flux crosses a wall
-            // face on any level (coarsening averages the zeros)
-            launch_zero_wall_faces(h->D0, h->L64[0].pa, h->stream);
-            check_launch();
-        }
-        for (int l = 1; l < h->nlev_p; ++l) {
-            launch_coarsen_coeffs<double>(h->L64[l - 1], h->L64[l], true, h->stream);
-            check_launch();
-        }
     }
     // BFBt: 1/diag(viscous operator) on faces, coarsened like 1/alpha
     if (h->knobs.visc_schur_approx == 1 && h->nlev_p > 0) {
         launch_inverse_diag_lap<double>(h->L64[0], h->knobs.visc_type, h->L64[0].pmu, h->stream);
         check_launch();
         for (int l = 1; l < h->nlev_p; ++l) {
-            LevelDev<double> F = h->L64[l - 1], C = h->L64[l];
-            for (int d = 0; d < 3; ++d) {
-                F.pa[d] = F.pmu[d];
-                C.pa[d] = C.pmu[d];
-            }
-            launch_coarsen_coeffs<double>(F, C, true, h->stream);
+            const LevelDev<double>&F = h->L64[l - 1], &C = h->L64[l];
+            launch_coarsen_faces<double>(F, C, F.pmu, C.pmu, h->stream);
             check_launch();
         }
     }
-    if (h->knobs.precision == LMM_PRECISION_FP32) {
-        for (int l = 0; l < (int)h->L64.size(); ++l) {
-            LevelDev<double>& a = h->L64[l];
-            LevelDev<float>& b = h->L32[l];
-            if (l < h->nlev) {
-                for (int d = 0; d < dm; ++d) launch_convert<double, float>(a.alpha[d], b.alpha[d], a.n, h->stream);
-                for (int e = 0; e < (dm == 2 ? 1 : 3); ++e)
-                    launch_convert<double, float>(a.bed[e], b.bed[e], edge_count(a.D, e), h->stream);
-                launch_convert<double, float>(a.beta, b.beta, a.n, h->stream);
-                launch_convert<double, float>(a.gamma, b.gamma, a.n, h->stream);
-            }
-            if (l < h->nlev_p)
-                for (int d = 0; d < dm; ++d) launch_convert<double, float>(a.pa[d], b.pa[d], a.n, h->stream);
-            if (l < h->nlev_p && h->knobs.visc_schur_approx == 1)
-                for (int d = 0; d < dm; ++d) launch_convert<double, float>(a.pmu[d], b.pmu[d], a.n, h->stream);
+    if (fp32 && h->knobs.visc_schur_approx == 1)
+        for (int l = 0; l < h->nlev_p; ++l) {
+            for (int d = 0; d < dm; ++d) launch_convert<double, float>(h->L64[l].pmu[d], h->L32[l].pmu[d], h->L64[l].n, h->stream);
             check_launch();
         }
-        for (int d = 0; d < dm; ++d) launch_convert<double, float>(h->alphainv[d], h->alphainv32[d], n, h->stream);
-        check_launch();
-    }
     // levels whose face coefficients are one value (constant density):
     // the pressure smoother and residual take 1/alpha as a scalar, the
-    // velocity operator theta*alpha (up to 16 levels of each; the flags
-    // and values share the handle's error word block and misc buffer)
+    // velocity operator theta*alpha (up to 16 levels of each)
     {
         const int np = std::min(h->nlev_p, 16), nv = std::min(h->nlev, 16);
-        int* flags = h->dev_err + 32;
-        LMM_CK(cudaMemsetAsync(flags, 0, 32 * sizeof(int), h->stream));
-        for (int l = 0; l < np; ++l) {
-            launch_uniform_check<double>(h->L64[l], flags + l, h->stream);
-            check_launch();
-            LMM_CK(cudaMemcpyAsync(h->hmisc + l, h->L64[l].pa[0], sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-        }
-        for (int l = 0; l < nv; ++l) {
-            launch_uniform_check<double>(h->L64[l], flags + 16 + l, h->stream, true);
-            check_launch();
-            LMM_CK(cudaMemcpyAsync(h->hmisc + 16 + l, h->L64[l].alpha[0], sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-        }
-        int* hflags = reinterpret_cast<int*>(h->hmisc + 32);
-        LMM_CK(cudaMemcpyAsync(hflags, flags, 32 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        LMM_CK(cudaMemcpyAsync(h->hmisc, h->ustate, 48 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        const int* hflags = reinterpret_cast<const int*>(h->hmisc + 32);
         LMM_CK(host_wait(h));
         std::vector<double> state;
         for (int l = 0; l < (int)h->L64.size(); ++l) {
@@ -1537,8 +1556,7 @@ int run_gmres(lmm_handle* h, double* theta_alpha, double* norm_pre_rhs, lmm_stat
     stokes_norm(h, h->tmp, 0);
     const double norm_pre_b = read_slot(h, 0, 5);
     if (norm_pre_rhs) *norm_pre_rhs = norm_pre_b;
-    stokes_norm(h, h->b, 0);
-    const double norm_b = read_slot(h, 0, 5);
+    const double norm_b = h->norm_b;
     if (st) {
         st->norm_b = norm_b;
         st->norm_pre_b = norm_pre_b;
@@ -1744,8 +1762,7 @@ int run_fgmres_augmented(lmm_handle* h, double* norm_pre_rhs, lmm_stats* st) {
     std::vector<int> zkind(mc + 1);  // 0: FP32 V-cycle column, 1: FP64 network column
     h->vcycles = 0;
     if (norm_pre_rhs) *norm_pre_rhs = 0.0;
-    stokes_norm(h, h->b, 0);
-    const double norm_b = read_slot(h, 0, 5);
+    const double norm_b = h->norm_b;
     if (st) st->norm_b = norm_b;
     if (!std::isfinite(norm_b)) return LMM_ERR_NONFINITE;
     if (norm_b <= 0.0) {
@@ -1927,8 +1944,7 @@ int run_fgmres(lmm_handle* h, double* norm_pre_rhs, lmm_stats* st, const FgmresR
         h->vcycles = 0;
         if (norm_pre_rhs) *norm_pre_rhs = 0.0;
     }
-    stokes_norm(h, h->b, 0);
-    const double norm_b = read_slot(h, 0, 5);
+    const double norm_b = h->norm_b;
     if (st) st->norm_b = norm_b;
     if (!std::isfinite(norm_b)) return LMM_ERR_NONFINITE;
     if (norm_b <= 0.0) {
@@ -2445,6 +2461,11 @@ static int create_impl(const lmm_grid* g, const lmm_knobs* k, int device, int ba
             h->alphainv[d] = h->alloc<double>(h->n);
             h->alphainv32[d] = h->alloc<float>(h->n);
         }
+        if (h->nlev_p > 0 && !h->D0.wall)
+            for (int d = 0; d < dm; ++d) {
+                h->L64[0].pa[d] = h->alphainv[d];
+                if (!h->L32.empty()) h->L32[0].pa[d] = h->alphainv32[d];
+            }
         for (int q = 0; q <= h->m; ++q) h->V.push_back(make_svec(h));
         if (k->method == LMM_METHOD_FGMRES) {
             for (int q = 0; q < h->m; ++q) {
@@ -2480,6 +2501,7 @@ static int create_impl(const lmm_grid* g, const lmm_knobs* k, int device, int ba
         h->partials = h->alloc<double>(partials_count(*g, batch));
         h->counter = h->alloc<unsigned>(std::max(64, batch));
         h->dev_err = h->alloc<int>(64);
+        h->ustate = h->alloc<double>(64);
         h->scal = h->alloc<double>(8 * lmm_handle::kSlots);
         int64_t st = 1;
         for (int d = 0; d < dm; ++d) st *= (g->n[d] + 1 + 8);
@@ -2622,19 +2644,33 @@ int solve_core(lmm_handle* h, const lmm_fields_in* in, const double* x0_u[3], co
     if (sf != 1.0) theta = theta * sf;
     LevelDev<double>& L0 = h->L64[0];
     // b = (scaled) rhs, x = (scaled) initial guess
-    for (int d = 0; d < dm; ++d) {
-        if (sf != 1.0)
-            launch_scale_copy<double>(in->b_u[d], h->b.c(d), sf, n, h->stream);
-        else
-            LMM_CK(cudaMemcpyAsync(h->b.c(d), in->b_u[d], n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-        LMM_CK(cudaMemcpyAsync(h->x.c(d), x0_u[d], n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+    {
+        CopyFields A{};
+        A.n = n;
+        int q = 0;
+        auto copy = [&](const double* src, double* dst) {
+            A.src[q] = src;
+            A.dst[q++] = dst;
+        };
+        for (int d = 0; d < dm; ++d) {
+            if (sf != 1.0) {
+                launch_scale_copy<double>(in->b_u[d], h->b.c(d), sf, n, h->stream);
+                check_launch();
+            } else {
+                copy(in->b_u[d], h->b.c(d));
+            }
+            copy(x0_u[d], h->x.c(d));
+        }
+        copy(in->b_p, h->b.p());
+        if (sf != 1.0) {
+            launch_scale_copy<double>(x0_p, h->x.p(), sf, n, h->stream);
+            check_launch();
+        } else {
+            copy(x0_p, h->x.p());
+        }
+        launch_copy_fields(A, q, h->stream);
+        check_launch();
     }
-    LMM_CK(cudaMemcpyAsync(h->b.p(), in->b_p, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    if (sf != 1.0)
-        launch_scale_copy<double>(x0_p, h->x.p(), sf, n, h->stream);
-    else
-        LMM_CK(cudaMemcpyAsync(h->x.p(), x0_p, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    check_launch();
     if (h->D0.wall) {
         // wall-normal velocities on the walls are not unknowns: zero in x
         // (apply_matrix's physbc_domainvel) and in b (the reference's
@@ -2664,7 +2700,11 @@ int solve_core(lmm_handle* h, const lmm_fields_in* in, const double* x0_u[3], co
         check_launch();
     }
     const double* al[3] = {in->alpha_fc[0], in->alpha_fc[1], in->alpha_fc[2]};
+    // |b|, read with the coefficient load's flags (one wait for both)
+    stokes_norm(h, h->b, 0);
+    LMM_CK(cudaMemcpyAsync(h->hscal, h->slot(0), 8 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     load_coeffs(h, al, beta, bed, gamma, theta);
+    h->norm_b = h->hscal[5];
     h->pvcycles = 0;
     int rc = (K.method == LMM_METHOD_FGMRES) ? run_fgmres(h, norm_pre_rhs, st) : run_gmres(h, theta_alpha, norm_pre_rhs, st);
     if (h->tma_smoother && rc != LMM_ERR_WATCHDOG) {
@@ -2704,9 +2744,16 @@ extern "C" int lmm_stokes_solve_device(lmm_handle* h, const lmm_fields_in* in, l
         const double* x0u[3] = {out->x_u[0], out->x_u[1], out->x_u[2]};
         int rc = solve_core(h, in, x0u, out->x_p, theta_alpha, norm_pre_rhs, st);
         if (rc >= 0 || rc == LMM_ERR_BREAKDOWN || rc == LMM_ERR_NONFINITE) {
-            for (int d = 0; d < h->dm; ++d)
-                LMM_CK(cudaMemcpyAsync(out->x_u[d], h->x.c(d), h->n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-            LMM_CK(cudaMemcpyAsync(out->x_p, h->x.p(), h->n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+            CopyFields A{};
+            A.n = h->n;
+            for (int d = 0; d < h->dm; ++d) {
+                A.src[d] = h->x.c(d);
+                A.dst[d] = out->x_u[d];
+            }
+            A.src[h->dm] = h->x.p();
+            A.dst[h->dm] = out->x_p;
+            launch_copy_fields(A, h->dm + 1, h->stream);
+            check_launch();
         }
         LMM_CK(cudaEventRecord(h->ev1, h->stream));
         LMM_CK(host_wait(h));
