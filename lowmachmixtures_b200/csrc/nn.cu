@@ -8,6 +8,7 @@
 #include "../../include/lmm_stokes.h"
 #include "kernels.h"
 #include "conv_tile_ws.cuh"
+#include "wgrad_tile.cuh"
 #include "nn_layers.cuh"
 #include "tc.cuh"
 
@@ -200,11 +201,44 @@ int conv3d(const bf16* x, const bf16* w, const float* bias, const bf16* skip, co
     return LMM_OK;
 }
 
+// the halo-tile weight gradient for NG groups of 8 input channels, NS output
+// channels per slice and P gradient planes per step: one CTA per SM (its
+// accumulators take the SM's TMEM), the steps split evenly
+template <int NG, int NS, int P>
+static int launch_wgrad_tile(WgradArgs A, int* err, cudaStream_t s) {
+    constexpr size_t smem = wg_smem_bytes(NG, NS, P);
+    static_assert(smem <= 227 * 1024, "operand stages fit in shared memory");
+    if (raise_smem_limit((const void*)k_conv3d_wgrad_tile<NG, NS, P>, smem) != cudaSuccess) return LMM_ERR_CUDA;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return LMM_ERR_CUDA;
+    A.tiles_x = (A.nx + kTX - 1) / kTX;
+    A.tiles_y = (A.ny + kTY - 1) / kTY;
+    A.zsteps = (A.nz + P - 1) / P;
+    const int64_t steps = (int64_t)A.tiles_x * A.tiles_y * A.zsteps * A.B;
+    if (steps > 0x7fffffff) return LMM_ERR_INVALID;
+    A.steps = (int)steps;
+    const int slices = (A.Cout + NS - 1) / NS;
+    const int per = std::max(1, sms / slices);
+    k_conv3d_wgrad_tile<NG, NS, P><<<dim3(A.steps < per ? A.steps : per, slices), kThreadsWG, smem, s>>>(A, err);
+    if (cudaGetLastError() != cudaSuccess) return LMM_ERR_CUDA;
+    count_launch();
+    return LMM_OK;
+}
+
 int conv3d_wgrad(const bf16* x, const bf16* g, float* dw, int B, int nx, int ny, int nz, int up, int Cin, int Cg, int Cout, int* err,
                  cudaStream_t s) {
     if (!x || !g || !dw || !err || B < 1 || Cin < 8 || (Cin % 8) || Cg < Cout || (Cg % 8) || Cout < 1 || Cout > 256 ||
         (up && ((nx | ny | nz) & 1)))
         return LMM_ERR_INVALID;
+    // the halo-tile kernel's channel counts (the network's), on any grid: 2531 -> 406 us for its
+    // eleven layers at 2 x 64^3; others the gathered GEMM
+    const WgradArgs T{x, g, dw, nx, ny, nz, up, B, Cg, Cout, 0, 0, 0, 0};
+    const bool wide = round_up(Cout, 16) % 32 == 0;   // 32-channel slices
+    if (Cin == 8) return launch_wgrad_tile<1, 16, 3>(T, err, s);
+    if (Cin == 16) return wide ? launch_wgrad_tile<2, 32, 1>(T, err, s) : launch_wgrad_tile<2, 16, 3>(T, err, s);
+    if (Cin == 32) return wide ? launch_wgrad_tile<4, 32, 1>(T, err, s) : launch_wgrad_tile<4, 16, 2>(T, err, s);
+    if (Cin == 64) return launch_wgrad_tile<8, 16, 1>(T, err, s);
     WgradGather G;
     G.x = x;
     G.gr = g;

@@ -130,6 +130,7 @@ static __global__ void __launch_bounds__(tc::kThreadsTC) k_conv3d(ConvGather G, 
 }
 
 // ------------------------------------------------------------ weight gradient
+// for channel counts without a halo-tile kernel (wgrad_tile.cuh: 8, 16, 32, 64)
 // dW[co][t][ci] += sum over this CTA's voxels of g[v][co] * x_tap_t(v)[ci];
 // rows of the GEMM are (t, ci), columns co, K the voxels.
 struct WgradGather {
