@@ -198,23 +198,23 @@ struct Net {
         rc |= wgrad(8, d1, g_c0, 16);
         rc |= dgrad(8, g_c0, nullptr, gup0);  // fine grid, 32 ch
         k_downsum<<<blocks_for(M(1) * 4), 256, 0, s>>>(gup0, tmp1, B, nx[1], ny[1], nz[1], 32);
-        k_grad_combine<<<blocks_for(M(1) * 32), 256, 0, s>>>(tmp1, nullptr, d1, g_d1, B, nx[1], ny[1], nz[1], 32);
+        k_grad_combine<<<blocks_for(M(1) * 4), 256, 0, s>>>(tmp1, nullptr, d1, g_d1, B, nx[1], ny[1], nz[1], 32);
         rc |= wgrad(7, c1, g_d1, 32);
         rc |= dgrad(7, g_d1, c1, g_c1);
         rc |= wgrad(6, b2, g_c1, 32);
         rc |= dgrad(6, g_c1, nullptr, gup1);  // level-1 grid, 64 ch
         k_downsum<<<blocks_for(M(2) * 8), 256, 0, s>>>(gup1, g_b2, B, nx[2], ny[2], nz[2], 64);
-        k_grad_combine<<<blocks_for(M(2) * 64), 256, 0, s>>>(g_b2, nullptr, b2, g_b2, B, nx[2], ny[2], nz[2], 64);
+        k_grad_combine<<<blocks_for(M(2) * 8), 256, 0, s>>>(g_b2, nullptr, b2, g_b2, B, nx[2], ny[2], nz[2], 64);
         rc |= wgrad(5, a2, g_b2, 64);
         rc |= dgrad(5, g_b2, a2, g_a2);
         rc |= wgrad(4, p1, g_a2, 64);
         rc |= dgrad(4, g_a2, nullptr, g_p1);  // level-2 grid, 32 ch
-        k_grad_combine<<<blocks_for(M(1) * 32), 256, 0, s>>>(g_c1, g_p1, s1, g_s1, B, nx[1], ny[1], nz[1], 32);
+        k_grad_combine<<<blocks_for(M(1) * 4), 256, 0, s>>>(g_c1, g_p1, s1, g_s1, B, nx[1], ny[1], nz[1], 32);
         rc |= wgrad(3, a1, g_s1, 32);
         rc |= dgrad(3, g_s1, a1, g_a1);
         rc |= wgrad(2, p0, g_a1, 32);
         rc |= dgrad(2, g_a1, nullptr, g_p0);  // level-1 grid, 16 ch
-        k_grad_combine<<<blocks_for(M(0) * 16), 256, 0, s>>>(g_c0, g_p0, s0, g_s0, B, nx[0], ny[0], nz[0], 16);
+        k_grad_combine<<<blocks_for(M(0) * 2), 256, 0, s>>>(g_c0, g_p0, s0, g_s0, B, nx[0], ny[0], nz[0], 16);
         rc |= wgrad(1, a0, g_s0, 16);
         rc |= dgrad(1, g_s0, a0, g_a0);
         rc |= wgrad(0, in, g_a0, 16);

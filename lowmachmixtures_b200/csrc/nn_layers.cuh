@@ -186,6 +186,14 @@ static __global__ void __launch_bounds__(tc::kThreadsTC) k_conv3d_wgrad(WgradGat
 }
 
 // ------------------------------------------------------------ elementwise
+__device__ __forceinline__ void unpack8_bf16(const uint4& u, float (&v)[8]) {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        v[2 * q] = __uint_as_float(w[q] << 16);
+        v[2 * q + 1] = __uint_as_float(w[q] & 0xFFFF0000u);
+    }
+}
 // the sum over the 8 fine children of coarse voxel (b, i, j, k), channels
 // 8g .. 8g+7, children in the order d = 0..7 (x fastest), in FP32; C % 8 == 0
 __device__ __forceinline__ void sum_children8(const bf16* __restrict__ f, int64_t b, int i, int j, int k, int g, int nx,
@@ -254,43 +262,66 @@ static __global__ void k_downsum(const bf16* __restrict__ f, bf16* __restrict__ 
 }
 
 // g = (a + pool_adjoint(p)) * (act > 0) on the fine grid [B][nz][ny][nx][C];
-// p (coarse, may be null) contributes p[parent] / 8
-static __global__ void k_grad_combine(const bf16* __restrict__ a, const bf16* __restrict__ p, const bf16* __restrict__ act,
-                               bf16* __restrict__ g, int B, int nx, int ny, int nz, int C) {
-    const int64_t n = (int64_t)B * nx * ny * nz * C;
+// p (coarse, may be null) contributes p[parent] / 8.  One thread per (voxel,
+// group of 8 channels), 16-byte loads (C % 8 == 0): bound by HBM, where one
+// thread per element was bound by its index divisions (16 channels at
+// 2 x 64^3 with p: 50 MB, 45 us).
+static __global__ void k_grad_combine(const bf16* a, const bf16* __restrict__ p, const bf16* __restrict__ act, bf16* g, int B, int nx,
+                                      int ny, int nz, int C) {
+    const int G = C / 8;
+    const int64_t n = (int64_t)B * nx * ny * nz * G;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-        float s = a ? __bfloat162float(a[e]) : 0.f;
+        float s[8] = {};
+        if (a) unpack8_bf16(reinterpret_cast<const uint4*>(a)[e], s);
         if (p) {
-            const int ch = (int)(e % C);
-            int64_t v = e / C;
+            const int q = (int)(e % G);
+            int64_t v = e / G;
             const int i = (int)(v % nx);
             v /= nx;
             const int j = (int)(v % ny);
             v /= ny;
             const int k = (int)(v % nz);
-            const int b = (int)(v / nz);
-            const int64_t pc = ((((int64_t)b * (nz / 2) + k / 2) * (ny / 2) + j / 2) * (nx / 2) + i / 2) * C + ch;
-            s += __bfloat162float(p[pc]) * 0.125f;
+            const int64_t b = v / nz;
+            float c[8];
+            unpack8_bf16(reinterpret_cast<const uint4*>(p)[(((b * (nz / 2) + k / 2) * (ny / 2) + j / 2) * (nx / 2) + i / 2) * G + q], c);
+#pragma unroll
+            for (int h = 0; h < 8; ++h) s[h] += c[h] * 0.125f;
         }
-        if (!(__bfloat162float(act[e]) > 0.f)) s = 0.f;
-        g[e] = __float2bfloat16(s);
+        float m[8];
+        unpack8_bf16(reinterpret_cast<const uint4*>(act)[e], m);
+#pragma unroll
+        for (int h = 0; h < 8; ++h)
+            if (!(m[h] > 0.f)) s[h] = 0.f;
+        reinterpret_cast<uint4*>(g)[e] = pack8_bf16(s, 1.f);
     }
 }
 
-// db[c] += sum_m g[m][c]  (Cs channels per row, the first C summed)
-static __global__ void k_bias_grad(const bf16* __restrict__ g, float* __restrict__ db, int64_t M, int C, int Cs) {
-    __shared__ float acc[64];
-    for (int c = threadIdx.x; c < 64; c += blockDim.x) acc[c] = 0.f;
+// db[c] += sum_m g[m][c]  (Cs channels per row, the first C summed).  A thread
+// sums one group of 8 channels (16-byte loads; its group is the same in every
+// pass), the lanes of a group by shuffles, the warps in shared memory.  Cs is 8,
+// 16, 32 or 64, blockDim.x 256.
+static __global__ void __launch_bounds__(256) k_bias_grad(const bf16* __restrict__ g, float* __restrict__ db, int64_t M, int C, int Cs) {
+    __shared__ float part[8][64];
+    const int G = Cs / 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float s[8] = {};
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < M * G; e += (int64_t)gridDim.x * blockDim.x) {
+        float v[8];
+        unpack8_bf16(reinterpret_cast<const uint4*>(g)[e], v);
+#pragma unroll
+        for (int h = 0; h < 8; ++h) s[h] += v[h];
+    }
+#pragma unroll
+    for (int h = 0; h < 8; ++h) {
+        for (int o = 16; o >= G; o >>= 1) s[h] += __shfl_xor_sync(0xffffffffu, s[h], o);
+        if (lane < G) part[warp][lane * 8 + h] = s[h];
+    }
     __syncthreads();
-    const int c = threadIdx.x % C;
-    const int lanes = blockDim.x / C;
-    float s = 0.f;
-    if ((int)threadIdx.x < lanes * C)
-        for (int64_t m = blockIdx.x * (int64_t)lanes + threadIdx.x / C; m < M; m += (int64_t)gridDim.x * lanes)
-            s += __bfloat162float(g[m * Cs + c]);
-    atomicAdd(&acc[c], s);
-    __syncthreads();
-    for (int q = threadIdx.x; q < C; q += blockDim.x) atomicAdd(&db[q], acc[q]);
+    for (int c = threadIdx.x; c < C; c += blockDim.x) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += part[w][c];
+        atomicAdd(&db[c], t);
+    }
 }
 
 // Adam on FP32 master parameters
