@@ -35,6 +35,8 @@ UNITS = [
     ("kernels_fp32.cu", ["-fmad=true"]),
     ("walls_fp64.cu", ["-fmad=false"]),
     ("walls_fp32.cu", ["-fmad=true"]),
+    ("leg_fp64.cu", ["-fmad=false"]),
+    ("leg_fp32.cu", ["-fmad=true"]),
     ("krylov.cu", ["-fmad=false"]),
     ("solver.cu", ["-fmad=false"]),
     ("coeffs.cu", ["-fmad=false"]),

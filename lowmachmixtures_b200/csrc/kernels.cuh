@@ -592,6 +592,19 @@ __device__ __forceinline__ T pcat(const T* a, const Dims& Dc, int i, int j, int 
         return cat<T, LD>(a, Dc, i, j, k);
 }
 
+// a b + c as the interpolation sums take it: FP32 fused on a periodic grid and
+// rounded twice on one with walls, FP64 rounded twice.  Written out, so a face
+// has the same bits in every kernel that interpolates it (left to the compiler,
+// a product that two sums share or that passes a wall rule is not contracted).
+template <bool W>
+__device__ __forceinline__ float madd(float a, float b, float c) {
+    return W ? __fadd_rn(__fmul_rn(a, b), c) : fmaf(a, b, c);
+}
+template <bool W>
+__device__ __forceinline__ double madd(double a, double b, double c) {
+    return __dadd_rn(__dmul_rn(a, b), c);
+}
+
 // v plus the interpolated coarse correction of the fine face of component
 // COMP at (i, j, k) (stag_prolongation's weights and order).  W: a fine wall
 // face keeps its zero (physbc_domainvel after the prolongation,
@@ -613,14 +626,13 @@ __device__ __forceinline__ T prolong_one(const Dims& Dc, const T* q, T v, int i,
         return pcat<T, LD, W, COMP>(q, Dc, y[0], y[1], y[2]);
     };
     if constexpr (DM == 2) {
-        if ((x[COMP] & 1) == 0) return v + T(0.75) * Q(0, 0, 0) + T(0.25) * Q(0, o1, 0);
-        return v + T(0.375) * Q(0, 0, 0) + T(0.125) * Q(0, o1, 0) + T(0.375) * Q(1, 0, 0) + T(0.125) * Q(1, o1, 0);
+        if ((x[COMP] & 1) == 0) return madd<W>(T(0.25), Q(0, o1, 0), madd<W>(T(0.75), Q(0, 0, 0), v));
+        return madd<W>(T(0.125), Q(1, o1, 0), madd<W>(T(0.375), Q(1, 0, 0), madd<W>(T(0.125), Q(0, o1, 0), madd<W>(T(0.375), Q(0, 0, 0), v))));
     } else {
         const T n16 = T(9.0 / 16.0), t16 = T(3.0 / 16.0), o16 = T(1.0 / 16.0);
         const T n32 = T(9.0 / 32.0), t32 = T(3.0 / 32.0), o32 = T(1.0 / 32.0);
-        if ((x[COMP] & 1) == 0) return v + n16 * Q(0, 0, 0) + t16 * Q(0, o1, 0) + t16 * Q(0, 0, o2) + o16 * Q(0, o1, o2);
-        return v + n32 * Q(0, 0, 0) + t32 * Q(0, o1, 0) + t32 * Q(0, 0, o2) + o32 * Q(0, o1, o2) + n32 * Q(1, 0, 0) +
-               t32 * Q(1, o1, 0) + t32 * Q(1, 0, o2) + o32 * Q(1, o1, o2);
+        if ((x[COMP] & 1) == 0) return madd<W>(o16, Q(0, o1, o2), madd<W>(t16, Q(0, 0, o2), madd<W>(t16, Q(0, o1, 0), madd<W>(n16, Q(0, 0, 0), v))));
+        return madd<W>(o32, Q(1, o1, o2), madd<W>(t32, Q(1, 0, o2), madd<W>(t32, Q(1, o1, 0), madd<W>(n32, Q(1, 0, 0), madd<W>(o32, Q(0, o1, o2), madd<W>(t32, Q(0, 0, o2), madd<W>(t32, Q(0, o1, 0), madd<W>(n32, Q(0, 0, 0), v))))))));
     }
 }
 
@@ -1333,17 +1345,6 @@ void launch_residual_restrict(const LevelDev<T>& F, const LevelDev<T>& Cc, int v
 }
 
 template <class T>
-void launch_prolong_add(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const phi_c[3], T* const phi_f[3],
-                        cudaStream_t s) {
-    if (F.D.wall) return wl_prolong_add<T>(F, Cc, phi_c, phi_f, s);
-    const G3 g = geom3_tuned(TK_PROLONG, sizeof(T), 0, F.D, F.D.nx, F.D.ny, F.D.nz);
-    if (F.D.dm == 2)
-        launch_pdl(k_prolong_add<T, 2>, g.grid, g.block, 0, s, F.D, Cc.D, phi_c[0], phi_c[1], phi_c[2], phi_f[0], phi_f[1], phi_f[2]);
-    else
-        launch_pdl(k_prolong_add<T, 3>, g.grid, g.block, 0, s, F.D, Cc.D, phi_c[0], phi_c[1], phi_c[2], phi_f[0], phi_f[1], phi_f[2]);
-}
-
-template <class T>
 void launch_coarsen_faces(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const f[3], T* const c[3], cudaStream_t s) {
     const G3 g = geom3(Cc.D.nx, Cc.D.ny, Cc.D.nz);
     if (F.D.dm == 2)
@@ -1548,7 +1549,6 @@ namespace lmm {
                                     cudaStream_t);                                                                             \
     template void launch_residual_restrict<T>(const LevelDev<T>&, const LevelDev<T>&, int, const T* const[3],                  \
                                               const T* const[3], T* const[3], cudaStream_t, int);                              \
-    template void launch_prolong_add<T>(const LevelDev<T>&, const LevelDev<T>&, const T* const[3], T* const[3], cudaStream_t); \
     template void launch_coarsen_faces<T>(const LevelDev<T>&, const LevelDev<T>&, const T* const[3], T* const[3], cudaStream_t); \
     template void launch_cc_smooth<T>(const LevelDev<T>&, int, cudaStream_t, int);                                              \
     template void launch_cc_residual_restrict<T>(const LevelDev<T>&, const LevelDev<T>&, cudaStream_t);                        \

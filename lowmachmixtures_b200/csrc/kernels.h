@@ -118,8 +118,6 @@ void wl_jacobi(const LevelDev<T>& L, int visc, const T* const rhs[3], const T* c
 template <class T>
 void wl_residual_restrict(const LevelDev<T>& F, const LevelDev<T>& Cc, int visc, const T* const rhs_f[3], const T* const phi_f[3],
                           T* const rhs_c[3], cudaStream_t s);
-template <class T>
-void wl_prolong_add(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const phi_c[3], T* const phi_f[3], cudaStream_t s);
 
 // The coarse end of a V-cycle (levels L[0..nl-1], L[0] already holding its
 // rhs) in one single-block launch with every level in shared memory
@@ -131,6 +129,16 @@ template <class T>
 cudaError_t launch_ccmg_tail(const LevelDev<T>* L, int nl, int nu1, int nu2, int nub, cudaStream_t s, bool zero);
 template <class T>
 size_t tail_smem_bytes(const LevelDev<T>* L, int nl, bool stag);
+
+// One level's leg of a V-cycle in one launch of a thread-block cluster
+// (leg.cuh).  Down: nsm smooths of L (zero: from phi = 0), the residual and
+// its restriction to Cc.rhs; up: the prolongation of Cc.phi and nsm smooths.
+// Gauss-Seidel levels of even sizes whose cells a cluster's threads can own.
+template <class T>
+bool leg_supported(const LevelDev<T>& L, int visc);
+template <class T>
+cudaError_t launch_level_leg(const LevelDev<T>& L, const LevelDev<T>& Cc, int visc, bool up, int nsm, double omega, cudaStream_t s,
+                             bool zero);
 
 // ---- pressure multigrid (this library's cell-centred V-cycle) ----
 // reverse: the launch takes the planes in decreasing order (same values)

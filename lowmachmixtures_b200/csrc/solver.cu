@@ -850,7 +850,7 @@ void autotune_levels(lmm_handle* h, std::vector<LevelDev<T>>& Ls) {
             if (kid == TK_APPLY_MATRIX && (l != 0 || h->batched || (sizeof(T) == 4 && h->Z32.empty()))) continue;
             const int kv = (kid == TK_PROLONG) ? 0 : visc;
             if (is_tuned(kid, sizeof(T), kv, L.D)) continue;
-            const int nxe = (kid == TK_GS_COLOUR) ? L.D.nx / 2 : L.D.nx;
+            const int nxe = (kid == TK_GS_COLOUR || kid == TK_PROLONG) ? L.D.nx / 2 : L.D.nx;
             auto launch = [&]() {
                 if (kid == TK_GS_COLOUR) {
                     for (int color = 1; color <= 2 * h->dm; ++color) {
@@ -930,6 +930,14 @@ int tail_start(lmm_handle* h, const std::vector<LevelDev<T>>& L, int nl, bool st
     return lc;
 }
 
+// the level's legs of a V-cycle run as cluster launches (leg.cuh)
+template <class T>
+bool use_leg(const lmm_handle* h, const LevelDev<T>& L) {
+    const lmm_knobs& K = h->knobs;
+    return K.tail_cells >= 0 && K.stag_mg_smoother != 0 && K.smoother_fusion <= 0 && K.residual_fusion <= 0 && !h->batched &&
+           !use_tma_smoother<T>(h, L) && leg_supported<T>(L, K.visc_type);
+}
+
 // one V-cycle on L[0].phi / L[0].rhs; zero: from L[0].phi = 0, whatever the
 // array holds (the coarse levels always start from zero)
 template <class T>
@@ -939,6 +947,11 @@ void vcycle(lmm_handle* h, std::vector<LevelDev<T>>& L, bool zero = false) {
     const int nl = h->nlev;
     const int lc = tail_start<T>(h, L, nl, true);
     for (int l = 0; l < lc && l < nl - 1; ++l) {
+        if (use_leg<T>(h, L[l])) {
+            LMM_CK(launch_level_leg<T>(L[l], L[l + 1], K.visc_type, false, K.stag_mg_nsmooths_down, K.stag_mg_omega, h->stream, l > 0 || zero));
+            check_launch();
+            continue;
+        }
         smooth<T>(h, L[l], K.stag_mg_nsmooths_down, l > 0 || zero);
         launch_residual_restrict<T>(L[l], L[l + 1], K.visc_type, L[l].rhs, L[l].phi, L[l + 1].rhs, h->stream,
                                     K.residual_fusion > 0 ? 1 : 0);
@@ -952,6 +965,11 @@ void vcycle(lmm_handle* h, std::vector<LevelDev<T>>& L, bool zero = false) {
         smooth<T>(h, L[nl - 1], K.stag_mg_nsmooths_bottom, nl > 1 || zero);
     }
     for (int l = std::min(lc, nl - 1) - 1; l >= 0; --l) {
+        if (use_leg<T>(h, L[l])) {
+            LMM_CK(launch_level_leg<T>(L[l], L[l + 1], K.visc_type, true, K.stag_mg_nsmooths_up, K.stag_mg_omega, h->stream, false));
+            check_launch();
+            continue;
+        }
         launch_prolong_add<T>(L[l], L[l + 1], L[l + 1].phi, L[l].phi, h->stream);
         check_launch();
         smooth<T>(h, L[l], K.stag_mg_nsmooths_up);

@@ -92,7 +92,7 @@ __device__ __forceinline__ bool bc_ok(const void* p, unsigned bytes) {
 // the translation units that include this header, each ending in
 // LMM_BC_UNIT(its name)
 #define LMM_BC_UNITS(X) \
-    X(autotune) X(coeffs) X(kernels_fp32) X(kernels_fp64) X(krylov) X(learned) X(net) X(nn) X(noalloc) X(solver) X(stochastic) X(walls_fp32) X(walls_fp64)
+    X(autotune) X(coeffs) X(kernels_fp32) X(kernels_fp64) X(krylov) X(learned) X(leg_fp32) X(leg_fp64) X(net) X(nn) X(noalloc) X(solver) X(stochastic) X(walls_fp32) X(walls_fp64)
 
 // neighbour offsets (with periodic wrap) of one index; 32-bit indices
 // (a field holds at most 2^31 - 1 entries)

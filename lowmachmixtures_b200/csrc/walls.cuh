@@ -110,15 +110,6 @@ void wl_residual_restrict(const LevelDev<T>& F, const LevelDev<T>& Cc, int visc,
         launch_pdl(k_restrict<T, 3, true>, gc.grid, gc.block, 0, s, F.D, F.tmp[0], F.tmp[1], F.tmp[2], Cc.D, rhs_c[0], rhs_c[1], rhs_c[2]);
 }
 
-template <class T>
-void wl_prolong_add(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const phi_c[3], T* const phi_f[3], cudaStream_t s) {
-    const G3 g = geom3(F.D.nx, F.D.ny, F.D.nz);
-    if (F.D.dm == 2)
-        launch_pdl(k_prolong_add<T, 2, true>, g.grid, g.block, 0, s, F.D, Cc.D, phi_c[0], phi_c[1], phi_c[2], phi_f[0], phi_f[1], phi_f[2]);
-    else
-        launch_pdl(k_prolong_add<T, 3, true>, g.grid, g.block, 0, s, F.D, Cc.D, phi_c[0], phi_c[1], phi_c[2], phi_f[0], phi_f[1], phi_f[2]);
-}
-
 #define LMM_INSTANTIATE_WALLS(T)                                                                                           \
     template void wl_gs_zero<T>(const LevelDev<T>&, int, const T* const[3], T* const[3], double, cudaStream_t); \
     template void wl_applyop<T>(const LevelDev<T>&, int, const T* const[3], T* const[3], cudaStream_t, int);              \
@@ -126,7 +117,6 @@ void wl_prolong_add(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* const 
     template void wl_jacobi<T>(const LevelDev<T>&, int, const T* const[3], const T* const[3], T* const[3], double,         \
                                cudaStream_t);                                                                              \
     template void wl_residual_restrict<T>(const LevelDev<T>&, const LevelDev<T>&, int, const T* const[3],                  \
-                                          const T* const[3], T* const[3], cudaStream_t);                                   \
-    template void wl_prolong_add<T>(const LevelDev<T>&, const LevelDev<T>&, const T* const[3], T* const[3], cudaStream_t);
+                                          const T* const[3], T* const[3], cudaStream_t);
 
 }  // namespace lmm
