@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "krylov.cuh"
+#include "cluster.cuh"
 #include "pdl.cuh"
 #include "stencil.cuh"
 
@@ -491,18 +492,52 @@ namespace {
 
 constexpr int kMdotThreads = 256;
 
-// The last block's sum of every block's partials, entry e of E: warp
-// e mod 8 takes it, its lanes stride over the blocks, then a shuffle tree
-// (a fixed order for a given grid).  The result goes to sh[e * ld].
-template <int E>
-__device__ __forceinline__ void sum_partials(const double* partials, double* sh, int ld) {
+// The sums over the blocks (of one instance) of E entries whose warps' sums are
+// in sh[e * kMdotThreads / 32 + warp]; true in the one block that goes on, with
+// entry e's sum in sh[e * kMdotThreads / 32].  The blocks' sums meet in global
+// memory and the last block to arrive adds them (CL: the grid is one cluster,
+// they meet in its first block's shared memory): warp e mod 8 takes entry e, its
+// lanes stride over the blocks, then a shuffle tree (a fixed order for a given grid).
+template <int E, bool CL>
+__device__ __forceinline__ bool grid_sums(double* sh, double* partials, unsigned* counter) {
+    constexpr int WARPS = kMdotThreads / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int e = warp; e < E; e += kMdotThreads / 32) {
-        double v = 0.0;
-        for (unsigned b = lane; b < gridDim.x; b += 32) v += ((volatile const double*)partials)[b * E + e];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) sh[e * ld] = v;
+    __syncthreads();
+    double mine = 0.0;
+    if (threadIdx.x < E)
+        for (int q = 0; q < WARPS; ++q) mine += sh[threadIdx.x * WARPS + q];
+    if constexpr (CL) {
+        __shared__ double meet[8][E];
+        cluster_wait();   // every block of the cluster runs
+        if (threadIdx.x < E) dsmem_store(dsmem_at((unsigned)__cvta_generic_to_shared(&meet[blockIdx.x][threadIdx.x]), 0), mine);
+        cluster_sync();
+        if (blockIdx.x != 0) return false;
+        for (int e = warp; e < E; e += WARPS) {
+            double v = lane < (int)gridDim.x ? meet[lane & 7][e] : 0.0;
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) sh[e * WARPS] = v;
+        }
+    } else {
+        __shared__ bool last;
+        if (threadIdx.x < E) {
+            partials[blockIdx.x * E + threadIdx.x] = mine;
+            __threadfence();
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+        __syncthreads();
+        if (!last) return false;
+        __threadfence();
+        for (int e = warp; e < E; e += WARPS) {
+            double v = 0.0;
+            for (unsigned b = lane; b < gridDim.x; b += 32) v += ((volatile const double*)partials)[b * E + e];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) sh[e * WARPS] = v;
+        }
+        if (threadIdx.x == 0) *counter = 0u;
     }
+    __syncthreads();
+    return true;
 }
 
 // Stokes inner products <w, V_k>, k < J, in one pass over w: per component
@@ -515,10 +550,11 @@ __device__ __forceinline__ void sum_partials(const double* partials, double* sh,
 // partitioned and summed as one problem alone.
 // (J = 5 held to three blocks per SM: unbounded, the compiler takes the
 // registers of two, and two blocks per SM keep too few loads in flight)
-template <int DM, int J>
+template <int DM, int J, bool CL>
 __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, const double* __restrict__ w, MVecs V, double wseam, double pw,
                                                        double* __restrict__ partials, unsigned* __restrict__ counter,
                                                        double* __restrict__ out, int64_t ss, int vec) {
+    if constexpr (CL) cluster_arrive();
     pdl_enter();
     constexpr int NC = DM + 1;
     const int n = D.nx * D.ny * (DM == 3 ? D.nz : 1);  // one instance
@@ -548,6 +584,7 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
         if constexpr (U == 1) {
             // per component: its J + 1 loads, then their products (the
             // compiler overlaps the next component's loads with them)
+#pragma unroll 2
             for (int p = tid; p < n2; p += stride) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
@@ -597,25 +634,31 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
             }
         }
     }
-    // seam planes of the face components (x: i == 0, y: j == 0, z: k == 0)
-#pragma unroll
-    for (int c = 0; c < DM; ++c) {
+    // seam planes of the face components (x: i == 0, y: j == 0, z: k == 0),
+    // the components' loads together
+    {
         const int nzi = (DM == 3) ? D.nz : 1;
-        const int m = (c == 0) ? D.ny * nzi : (c == 1 ? D.nx * nzi : D.nx * D.ny);
-        double v[J];
+        const int m[3] = {D.ny * nzi, D.nx * nzi, D.nx * D.ny};
+        const int most = DM == 3 ? max(m[0], max(m[1], m[2])) : max(m[0], m[1]);
+        double v[DM][J];
 #pragma unroll
-        for (int k = 0; k < J; ++k) v[k] = 0.0;
-        for (int q = tid; q < m; q += stride) {
-            int t;
-            if (c == 0) t = D.nx * q;
-            else if (c == 1) t = (q % D.nx) + D.nx * D.ny * (q / D.nx);
-            else t = q;
-            const double x = __ldg(w + (int64_t)c * N + t);
+        for (int c = 0; c < DM; ++c)
 #pragma unroll
-            for (int k = 0; k < J; ++k) v[k] += x * __ldg(V.p[k] + (int64_t)c * N + t);
+            for (int k = 0; k < J; ++k) v[c][k] = 0.0;
+        for (int q = tid; q < most; q += stride) {
+            const int t[3] = {D.nx * q, (q % D.nx) + D.nx * D.ny * (q / D.nx), q};
+#pragma unroll
+            for (int c = 0; c < DM; ++c) {
+                if (q >= m[c]) continue;
+                const double x = __ldg(w + (int64_t)c * N + t[c]);
+#pragma unroll
+                for (int k = 0; k < J; ++k) v[c][k] += x * __ldg(V.p[k] + (int64_t)c * N + t[c]);
+            }
         }
 #pragma unroll
-        for (int k = 0; k < J; ++k) acc[k][c] += (wseam - 1.0) * v[k];
+        for (int c = 0; c < DM; ++c)
+#pragma unroll
+            for (int k = 0; k < J; ++k) acc[k][c] += (wseam - 1.0) * v[c][k];
     }
     __shared__ double sh[J * NC][kMdotThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -627,28 +670,13 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
             if (lane == 0) sh[k * NC + c][warp] = v;
         }
-    __syncthreads();
-    if (threadIdx.x < J * NC) {
-        double v = 0.0;
-        for (int q = 0; q < kMdotThreads / 32; ++q) v += sh[threadIdx.x][q];
-        partials[blockIdx.x * J * NC + threadIdx.x] = v;
-    }
-    __threadfence();
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    sum_partials<J * NC>(partials, &sh[0][0], kMdotThreads / 32);
-    __syncthreads();
+    if (!grid_sums<J * NC, CL>(&sh[0][0], partials, counter)) return;
     if (threadIdx.x < J) {
         const int k = threadIdx.x;
         double su = 0.0;
         for (int c = 0; c < DM; ++c) su = su + sh[k * NC + c][0];
         out[k * ss + 4] = su + (pw * pw) * sh[k * NC + DM][0];
     }
-    if (threadIdx.x == 0) *counter = 0u;
 }
 
 // w -= sum_k h_k V_k, h_k = hs[k * ss + 4] (a 2D batch: the entry's
@@ -668,11 +696,12 @@ __global__ void k_maxpy(double* __restrict__ w, MVecs V, const double* __restric
 // w -= sum_k h_k V_k (as k_maxpy) and, in the same pass, the Stokes norm of
 // the new w with the seam weight applied per entry: out[5] = sqrt(|u|^2 +
 // (pw |p|)^2), out[4] the squared form (as k_reduce's slots)
-template <int DM, int J>
+template <int DM, int J, bool CL>
 __global__ void __launch_bounds__(kMdotThreads) k_maxpy_norm(Dims D, double* __restrict__ w, MVecs V, const double* __restrict__ hs,
                                                              double wseam, double pw, double* __restrict__ partials,
                                                              unsigned* __restrict__ counter, double* __restrict__ out, int64_t ss,
                                                              int vec) {
+    if constexpr (CL) cluster_arrive();
     pdl_enter();
     constexpr int NC = DM + 1;
     const int n = D.nx * D.ny * (DM == 3 ? D.nz : 1);  // one instance (blockIdx.y, as k_mdot)
@@ -746,28 +775,13 @@ __global__ void __launch_bounds__(kMdotThreads) k_maxpy_norm(Dims D, double* __r
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         if (lane == 0) sh[c][warp] = v;
     }
-    __syncthreads();
-    if (threadIdx.x < NC) {
-        double v = 0.0;
-        for (int q = 0; q < kMdotThreads / 32; ++q) v += sh[threadIdx.x][q];
-        partials[blockIdx.x * NC + threadIdx.x] = v;
-    }
-    __threadfence();
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    sum_partials<NC>(partials, &sh[0][0], kMdotThreads / 32);
-    __syncthreads();
+    if (!grid_sums<NC, CL>(&sh[0][0], partials, counter)) return;
     if (threadIdx.x == 0) {
         double su = 0.0;
         for (int c = 0; c < DM; ++c) su = su + sh[c][0];
         out[4] = su + (pw * pw) * sh[DM][0];
         const double nu = sqrt(su), np = pw * sqrt(sh[DM][0]);
         out[5] = sqrt(nu * nu + np * np);
-        *counter = 0u;
     }
 }
 
@@ -776,6 +790,8 @@ __global__ void __launch_bounds__(kMdotThreads) k_maxpy_norm(Dims D, double* __r
 namespace {
 template <int DM, int J, bool NORM>
 int cgs_blocks(int64_t n);
+// blocks of the cluster variant (the grid of one instance is one cluster), 0: too many
+int cgs_cluster(int64_t n) { return mdot_blocks(n) <= 8 ? mdot_blocks(n) : 0; }
 // the Gram-Schmidt passes may take entries in pairs: rows of even length
 // (no pair straddles a row or an instance) and 16-byte aligned vectors
 int pairs_ok(const Dims& D, const void* w, const MVecs& V, int J) {
@@ -789,7 +805,12 @@ void launch_maxpy_norm(const Dims& D, double* w, const MVecs& V, int J, const do
                        unsigned* counter, double* out, cudaStream_t s, int ninst, int64_t ss) {
     const int64_t n = (int64_t)D.nx * D.ny * (D.dm == 3 ? D.nz : 1);
     const int vec = pairs_ok(D, w, V, J);
-#define MN(DM_, J_) launch_pdl(k_maxpy_norm<DM_, J_>, dim3(cgs_blocks<DM_, J_, true>(n), ninst), dim3(kMdotThreads), 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec)
+    const int cl = cgs_cluster(n);
+#define MN(DM_, J_)                                                                                                     \
+    if (cl)                                                                                                             \
+        launch_cluster(k_maxpy_norm<DM_, J_, true>, dim3(cl, ninst), dim3(kMdotThreads), cl, 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec); \
+    else                                                                                                                \
+        launch_pdl(k_maxpy_norm<DM_, J_, false>, dim3(cgs_blocks<DM_, J_, true>(n), ninst), dim3(kMdotThreads), 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec)
 #define MNJ(DM_)                               \
     switch (J) {                               \
     case 1: MN(DM_, 1); break;                 \
@@ -822,7 +843,7 @@ int cgs_blocks(int64_t n) {
         int dev = 0, sms = 148, per_sm = 4;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const void* k = NORM ? (const void*)k_maxpy_norm<DM, J> : (const void*)k_mdot<DM, J>;
+        const void* k = NORM ? (const void*)k_maxpy_norm<DM, J, false> : (const void*)k_mdot<DM, J, false>;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kMdotThreads, 0) != cudaSuccess || per_sm < 1) {
             cudaGetLastError();
             per_sm = 1;
@@ -837,7 +858,12 @@ void launch_mdot(const Dims& D, const double* w, const MVecs& V, int J, double w
                  double* out, cudaStream_t s, int ninst, int64_t ss) {
     const int64_t n = (int64_t)D.nx * D.ny * (D.dm == 3 ? D.nz : 1);
     const int vec = pairs_ok(D, w, V, J);
-#define MD(DM_, J_) launch_pdl(k_mdot<DM_, J_>, dim3(cgs_blocks<DM_, J_, false>(n), ninst), dim3(kMdotThreads), 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec)
+    const int cl = cgs_cluster(n);
+#define MD(DM_, J_)                                                                                                     \
+    if (cl)                                                                                                             \
+        launch_cluster(k_mdot<DM_, J_, true>, dim3(cl, ninst), dim3(kMdotThreads), cl, 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec); \
+    else                                                                                                                \
+        launch_pdl(k_mdot<DM_, J_, false>, dim3(cgs_blocks<DM_, J_, false>(n), ninst), dim3(kMdotThreads), 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec)
 #define MDJ(DM_)                               \
     switch (J) {                               \
     case 1: MD(DM_, 1); break;                 \

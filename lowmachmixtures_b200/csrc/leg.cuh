@@ -41,24 +41,6 @@ struct LegArgs {
     T* crhs[3];              // down: the coarse right-hand side
 };
 
-__device__ __forceinline__ void cluster_sync() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// the address of shared-memory byte `a` of the CTA with rank r
-__device__ __forceinline__ unsigned dsmem_at(unsigned a, unsigned r) {
-    unsigned o;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(r));
-    return o;
-}
-__device__ __forceinline__ void dsmem_store(unsigned a, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
-__device__ __forceinline__ void dsmem_store(unsigned a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
-
 // A cell a thread owns.  phi of the slab is stored by parity of i + j + k, each
 // half densely along pairs (2h, 2h + 1), so the lanes of a warp read and write
 // consecutive words whichever colour they are on (interleaved, every access had
@@ -345,20 +327,7 @@ static cudaError_t launch_leg_k(K kernel, const A& args, const LegShape& sh, int
         e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks * sh.nc);
-    cfg.blockDim = dim3(sh.threads);
-    cfg.dynamicSmemBytes = sh.smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = sh.nc;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, kernel, args);
+    return launch_cluster(kernel, dim3(blocks * sh.nc), dim3(sh.threads), sh.nc, sh.smem, s, args);
 }
 
 template <class T, int DM, bool W, int PP>
