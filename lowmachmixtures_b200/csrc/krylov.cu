@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
         if constexpr (U == 1) {
             // per component: its J + 1 loads, then their products (the
             // compiler overlaps the next component's loads with them)
-#pragma unroll 2
+#pragma unroll(CL ? 2 : 1)
             for (int p = tid; p < n2; p += stride) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
@@ -634,11 +634,13 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
             }
         }
     }
-    // seam planes of the face components (x: i == 0, y: j == 0, z: k == 0),
-    // the components' loads together
-    {
-        const int nzi = (DM == 3) ? D.nz : 1;
-        const int m[3] = {D.ny * nzi, D.nx * nzi, D.nx * D.ny};
+    // seam planes of the face components (x: i == 0, y: j == 0, z: k == 0); CL:
+    // the components' loads together (in a large grid their registers would
+    // cost resident blocks)
+    const int nzi = (DM == 3) ? D.nz : 1;
+    const int m[3] = {D.ny * nzi, D.nx * nzi, D.nx * D.ny};
+    auto seam = [&](int c, int q) { return c == 0 ? D.nx * q : (c == 1 ? (q % D.nx) + D.nx * D.ny * (q / D.nx) : q); };
+    if constexpr (CL) {
         const int most = DM == 3 ? max(m[0], max(m[1], m[2])) : max(m[0], m[1]);
         double v[DM][J];
 #pragma unroll
@@ -646,19 +648,33 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
 #pragma unroll
             for (int k = 0; k < J; ++k) v[c][k] = 0.0;
         for (int q = tid; q < most; q += stride) {
-            const int t[3] = {D.nx * q, (q % D.nx) + D.nx * D.ny * (q / D.nx), q};
 #pragma unroll
             for (int c = 0; c < DM; ++c) {
                 if (q >= m[c]) continue;
-                const double x = __ldg(w + (int64_t)c * N + t[c]);
+                const double x = __ldg(w + (int64_t)c * N + seam(c, q));
 #pragma unroll
-                for (int k = 0; k < J; ++k) v[c][k] += x * __ldg(V.p[k] + (int64_t)c * N + t[c]);
+                for (int k = 0; k < J; ++k) v[c][k] += x * __ldg(V.p[k] + (int64_t)c * N + seam(c, q));
             }
         }
 #pragma unroll
         for (int c = 0; c < DM; ++c)
 #pragma unroll
             for (int k = 0; k < J; ++k) acc[k][c] += (wseam - 1.0) * v[c][k];
+    } else {
+#pragma unroll
+        for (int c = 0; c < DM; ++c) {
+            double v[J];
+#pragma unroll
+            for (int k = 0; k < J; ++k) v[k] = 0.0;
+            for (int q = tid; q < m[c]; q += stride) {
+                const int t = seam(c, q);
+                const double x = __ldg(w + (int64_t)c * N + t);
+#pragma unroll
+                for (int k = 0; k < J; ++k) v[k] += x * __ldg(V.p[k] + (int64_t)c * N + t);
+            }
+#pragma unroll
+            for (int k = 0; k < J; ++k) acc[k][c] += (wseam - 1.0) * v[k];
+        }
     }
     __shared__ double sh[J * NC][kMdotThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
