@@ -130,6 +130,11 @@ cudaError_t launch_ccmg_tail(const LevelDev<T>* L, int nl, int nu1, int nu2, int
 template <class T>
 size_t tail_smem_bytes(const LevelDev<T>* L, int nl, bool stag);
 
+// out = the residual (L phi - rhs) * -1 by pairs of cells (pair3.cuh); false:
+// not a level or arrays that it takes, nothing launched
+template <class T>
+bool launch_residual_pairs(const LevelDev<T>& L, int visc, const T* const rhs[3], const T* const phi[3], T* const out[3], cudaStream_t s);
+
 // One level's leg of a V-cycle in one launch of a thread-block cluster
 // (leg.cuh).  Down: nsm smooths of L (zero: from phi = 0), the residual and
 // its restriction to Cc.rhs; up: the prolongation of Cc.phi and nsm smooths.

@@ -4,6 +4,7 @@
 
 #include "krylov.cuh"
 #include "cluster.cuh"
+#include "pair3.cuh"
 #include "pdl.cuh"
 #include "stencil.cuh"
 
@@ -78,6 +79,13 @@ template <class TX>
 static void apply_matrix_impl(const LevelDev<double>& L0, int visc, const TX* const x[4], double* const b[4], cudaStream_t s) {
     const double dxsqinv = 1.0 / (L0.dx * L0.dx);
     const double dxinv = 1.0 / L0.dx;
+    if (L0.D.dm == 3 && pairs_supported<double>(L0.D, L0.coef(), visc, x, 4, b, 4)) {
+        const dim3 pb = pair_block(L0.D, TK_APPLY_MATRIX, sizeof(TX), visc), pg = pair_grid(L0.D, pb);
+#define AMP(V_) launch_pdl(k_apply_matrix_pairs<V_, TX>, pg, pb, 0, s, L0.D, L0.coef(), x[0], x[1], x[2], x[3], b[0], b[1], b[2], b[3], dxsqinv, dxinv)
+        if (visc == -1) AMP(-1); else if (visc == -2) AMP(-2); else AMP(-3);
+#undef AMP
+        return;
+    }
     // periodic grids: the block shape the autotuner chose (a shape it
     // forces while it times them), else 64 x 4
     Shape sh = forced_shape();

@@ -21,6 +21,7 @@
 // one pair a thread and 0.9 with two, where the SM's issue slots bound it; more
 // cells than that (leg_shape) keep their launches.
 #pragma once
+#include "pair3.cuh"
 #include "prolong.cuh"
 #include "tail.cuh"
 
@@ -381,6 +382,7 @@ cudaError_t launch_level_leg(const LevelDev<T>& L, const LevelDev<T>& Cc, int vi
 
 #define LMM_INSTANTIATE_LEG(T)                                                  \
     template bool leg_supported<T>(const LevelDev<T>&, int);                    \
+    template bool launch_residual_pairs<T>(const LevelDev<T>&, int, const T* const[3], const T* const[3], T* const[3], cudaStream_t); \
     template void launch_prolong_add<T>(const LevelDev<T>&, const LevelDev<T>&, const T* const[3], T* const[3], cudaStream_t); \
     template cudaError_t launch_level_leg<T>(const LevelDev<T>&, const LevelDev<T>&, int, bool, int, double, cudaStream_t, bool);
 

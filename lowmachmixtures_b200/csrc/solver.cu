@@ -850,7 +850,10 @@ void autotune_levels(lmm_handle* h, std::vector<LevelDev<T>>& Ls) {
             if (kid == TK_APPLY_MATRIX && (l != 0 || h->batched || (sizeof(T) == 4 && h->Z32.empty()))) continue;
             const int kv = (kid == TK_PROLONG) ? 0 : visc;
             if (is_tuned(kid, sizeof(T), kv, L.D)) continue;
-            const int nxe = (kid == TK_GS_COLOUR || kid == TK_PROLONG) ? L.D.nx / 2 : L.D.nx;
+            // kernels with a thread per pair of a row; those of pair3.cuh take at most 128 threads
+            const bool pair3 = L.D.dm == 3 && visc < 0 &&
+                               (kid == TK_APPLY_MATRIX || (kid == TK_RESIDUAL && (sizeof(T) == 8 || visc == -2)));
+            const int nxe = (kid == TK_GS_COLOUR || kid == TK_PROLONG || pair3) ? L.D.nx / 2 : L.D.nx;
             auto launch = [&]() {
                 if (kid == TK_GS_COLOUR) {
                     for (int color = 1; color <= 2 * h->dm; ++color) {
@@ -874,7 +877,7 @@ void autotune_levels(lmm_handle* h, std::vector<LevelDev<T>>& Ls) {
             double best = 1e300, def = 0.0;
             Shape bs{};
             for (const Shape& c : cands) {
-                if (c.bx > std::max(nxe, 32)) continue;
+                if (c.bx > std::max(nxe, 32) || (pair3 && c.bx * c.by > 128)) continue;
                 force_shape(c);
                 launch();
                 constexpr int kReps = 5;
