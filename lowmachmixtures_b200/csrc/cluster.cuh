@@ -35,9 +35,9 @@ __device__ __forceinline__ unsigned dsmem_at(unsigned a, unsigned r) {
 __device__ __forceinline__ void dsmem_store(unsigned a, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
 __device__ __forceinline__ void dsmem_store(unsigned a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
 
-// clusters of nc blocks along x (grid.x a multiple of nc)
+// clusters of nc.x x nc.y x nc.z blocks, ranked x fastest (each extent of the grid a multiple of its)
 template <class... KArgs, class... Args>
-static inline cudaError_t launch_cluster(void (*k)(KArgs...), dim3 grid, dim3 block, int nc, size_t smem, cudaStream_t s, Args... args) {
+static inline cudaError_t launch_cluster(void (*k)(KArgs...), dim3 grid, dim3 block, dim3 nc, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -47,8 +47,9 @@ static inline cudaError_t launch_cluster(void (*k)(KArgs...), dim3 grid, dim3 bl
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = nc;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    at[1].val.clusterDim.x = nc.x;
+    at[1].val.clusterDim.y = nc.y;
+    at[1].val.clusterDim.z = nc.z;
     cfg.attrs = at;
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, k, args...);

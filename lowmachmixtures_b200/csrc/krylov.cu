@@ -506,20 +506,22 @@ constexpr int kMdotThreads = 256;
 // memory and the last block to arrive adds them (CL: the grid is one cluster,
 // they meet in its first block's shared memory): warp e mod 8 takes entry e, its
 // lanes stride over the blocks, then a shuffle tree (a fixed order for a given grid).
-template <int E, bool CL>
-__device__ __forceinline__ bool grid_sums(double* sh, double* partials, unsigned* counter) {
+// mine(e): entry e is summed by this block (a grid split by component: blockIdx.z).
+template <int E, bool CL, class Mine>
+__device__ __forceinline__ bool grid_sums(double* sh, double* partials, unsigned* counter, Mine mine) {
     constexpr int WARPS = kMdotThreads / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __syncthreads();
-    double mine = 0.0;
-    if (threadIdx.x < E)
-        for (int q = 0; q < WARPS; ++q) mine += sh[threadIdx.x * WARPS + q];
+    double sum = 0.0;
+    const bool has = threadIdx.x < E && mine(threadIdx.x);
+    if (has)
+        for (int q = 0; q < WARPS; ++q) sum += sh[threadIdx.x * WARPS + q];
     if constexpr (CL) {
         __shared__ double meet[8][E];
         cluster_wait();   // every block of the cluster runs
-        if (threadIdx.x < E) dsmem_store(dsmem_at((unsigned)__cvta_generic_to_shared(&meet[blockIdx.x][threadIdx.x]), 0), mine);
+        if (has) dsmem_store(dsmem_at((unsigned)__cvta_generic_to_shared(&meet[blockIdx.x][threadIdx.x]), 0), sum);
         cluster_sync();
-        if (blockIdx.x != 0) return false;
+        if (cluster_rank() != 0) return false;
         for (int e = warp; e < E; e += WARPS) {
             double v = lane < (int)gridDim.x ? meet[lane & 7][e] : 0.0;
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -527,12 +529,12 @@ __device__ __forceinline__ bool grid_sums(double* sh, double* partials, unsigned
         }
     } else {
         __shared__ bool last;
-        if (threadIdx.x < E) {
-            partials[blockIdx.x * E + threadIdx.x] = mine;
+        if (has) {
+            partials[blockIdx.x * E + threadIdx.x] = sum;
             __threadfence();
         }
         __syncthreads();
-        if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+        if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == gridDim.x * gridDim.z - 1);
         __syncthreads();
         if (!last) return false;
         __threadfence();
@@ -558,7 +560,7 @@ __device__ __forceinline__ bool grid_sums(double* sh, double* partials, unsigned
 // partitioned and summed as one problem alone.
 // (J = 5 held to three blocks per SM: unbounded, the compiler takes the
 // registers of two, and two blocks per SM keep too few loads in flight)
-template <int DM, int J, bool CL>
+template <int DM, int J, bool CL, bool CS>
 __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, const double* __restrict__ w, MVecs V, double wseam, double pw,
                                                        double* __restrict__ partials, unsigned* __restrict__ counter,
                                                        double* __restrict__ out, int64_t ss, int vec) {
@@ -581,6 +583,7 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
     for (int k = 0; k < J; ++k)
 #pragma unroll
         for (int c = 0; c < NC; ++c) acc[k][c] = 0.0;
+    auto mine = [&](int c) { return !CS || c == (int)blockIdx.z; };   // a component this block sums
     const int stride = gridDim.x * blockDim.x;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     if (vec) {
@@ -592,10 +595,11 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
         if constexpr (U == 1) {
             // per component: its J + 1 loads, then their products (the
             // compiler overlaps the next component's loads with them)
-#pragma unroll(CL ? 2 : 1)
+#pragma unroll(CL || CS ? 2 : 1)
             for (int p = tid; p < n2; p += stride) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
+                    if (!mine(c)) continue;
                     const double2 x = __ldg(reinterpret_cast<const double2*>(w + (int64_t)c * N) + p);
                     double2 v[J];
 #pragma unroll
@@ -615,6 +619,7 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
                 const int p = min(p0 + u * stride, n2 - 1);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
+                    if (!mine(c)) continue;
                     x[u][c] = __ldg(reinterpret_cast<const double2*>(w + (int64_t)c * N) + p);
 #pragma unroll
                     for (int k = 0; k < J; ++k) v[u][k][c] = __ldg(reinterpret_cast<const double2*>(V.p[k] + (int64_t)c * N) + p);
@@ -624,18 +629,21 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
             for (int u = 0; u < U; ++u) {
                 if (u > 0 && p0 + u * stride >= n2) break;
 #pragma unroll
-                for (int c = 0; c < NC; ++c)
+                for (int c = 0; c < NC; ++c) {
+                    if (!mine(c)) continue;
 #pragma unroll
                     for (int k = 0; k < J; ++k) {
                         acc[k][c] += x[u][c].x * v[u][k][c].x;
                         acc[k][c] += x[u][c].y * v[u][k][c].y;
                     }
+                }
             }
         }
     } else {
         for (int t = tid; t < n; t += stride) {
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
+                if (!mine(c)) continue;
                 const double x = __ldg(w + (int64_t)c * N + t);
 #pragma unroll
                 for (int k = 0; k < J; ++k) acc[k][c] += x * __ldg(V.p[k] + (int64_t)c * N + t);
@@ -648,7 +656,7 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
     const int nzi = (DM == 3) ? D.nz : 1;
     const int m[3] = {D.ny * nzi, D.nx * nzi, D.nx * D.ny};
     auto seam = [&](int c, int q) { return c == 0 ? D.nx * q : (c == 1 ? (q % D.nx) + D.nx * D.ny * (q / D.nx) : q); };
-    if constexpr (CL) {
+    if constexpr (CL || CS) {
         const int most = DM == 3 ? max(m[0], max(m[1], m[2])) : max(m[0], m[1]);
         double v[DM][J];
 #pragma unroll
@@ -658,7 +666,7 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
         for (int q = tid; q < most; q += stride) {
 #pragma unroll
             for (int c = 0; c < DM; ++c) {
-                if (q >= m[c]) continue;
+                if (q >= m[c] || !mine(c)) continue;
                 const double x = __ldg(w + (int64_t)c * N + seam(c, q));
 #pragma unroll
                 for (int k = 0; k < J; ++k) v[c][k] += x * __ldg(V.p[k] + (int64_t)c * N + seam(c, q));
@@ -671,6 +679,7 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
     } else {
 #pragma unroll
         for (int c = 0; c < DM; ++c) {
+            if (!mine(c)) continue;
             double v[J];
 #pragma unroll
             for (int k = 0; k < J; ++k) v[k] = 0.0;
@@ -690,11 +699,12 @@ __global__ void __launch_bounds__(kMdotThreads, J == 5 ? 3 : 0) k_mdot(Dims D, c
     for (int k = 0; k < J; ++k)
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
+            if (!mine(c)) continue;
             double v = acc[k][c];
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
             if (lane == 0) sh[k * NC + c][warp] = v;
         }
-    if (!grid_sums<J * NC, CL>(&sh[0][0], partials, counter)) return;
+    if (!grid_sums<J * NC, CL>(&sh[0][0], partials, counter, [&](int e) { return mine(e % NC); })) return;
     if (threadIdx.x < J) {
         const int k = threadIdx.x;
         double su = 0.0;
@@ -720,7 +730,7 @@ __global__ void k_maxpy(double* __restrict__ w, MVecs V, const double* __restric
 // w -= sum_k h_k V_k (as k_maxpy) and, in the same pass, the Stokes norm of
 // the new w with the seam weight applied per entry: out[5] = sqrt(|u|^2 +
 // (pw |p|)^2), out[4] the squared form (as k_reduce's slots)
-template <int DM, int J, bool CL>
+template <int DM, int J, bool CL, bool CS>
 __global__ void __launch_bounds__(kMdotThreads) k_maxpy_norm(Dims D, double* __restrict__ w, MVecs V, const double* __restrict__ hs,
                                                              double wseam, double pw, double* __restrict__ partials,
                                                              unsigned* __restrict__ counter, double* __restrict__ out, int64_t ss,
@@ -746,6 +756,7 @@ __global__ void __launch_bounds__(kMdotThreads) k_maxpy_norm(Dims D, double* __r
     double acc[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+    auto mine = [&](int c) { return !CS || c == (int)blockIdx.z; };   // a component this block updates
     const int stride = gridDim.x * blockDim.x;
     if (vec) {
         // entry pairs (2p, 2p+1) of one row by 16-byte loads and stores
@@ -757,12 +768,14 @@ __global__ void __launch_bounds__(kMdotThreads) k_maxpy_norm(Dims D, double* __r
             double2 x[NC], v[J][NC];
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
+                if (!mine(c)) continue;
                 x[c] = reinterpret_cast<const double2*>(w + (int64_t)c * N)[p];
 #pragma unroll
                 for (int k = 0; k < J; ++k) v[k][c] = __ldg(reinterpret_cast<const double2*>(V.p[k] + (int64_t)c * N) + p);
             }
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
+                if (!mine(c)) continue;
 #pragma unroll
                 for (int k = 0; k < J; ++k) {
                     x[c].x = x[c].x - v[k][c].x * h[k];
@@ -781,6 +794,7 @@ __global__ void __launch_bounds__(kMdotThreads) k_maxpy_norm(Dims D, double* __r
             const int i = t % D.nx, r = t / D.nx, j = r % D.ny, kk = r / D.ny;
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
+                if (!mine(c)) continue;
                 const int64_t e = (int64_t)c * N + t;
                 double x = w[e];
 #pragma unroll
@@ -795,11 +809,12 @@ __global__ void __launch_bounds__(kMdotThreads) k_maxpy_norm(Dims D, double* __r
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
+        if (!mine(c)) continue;
         double v = acc[c];
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         if (lane == 0) sh[c][warp] = v;
     }
-    if (!grid_sums<NC, CL>(&sh[0][0], partials, counter)) return;
+    if (!grid_sums<NC, CL>(&sh[0][0], partials, counter, mine)) return;
     if (threadIdx.x == 0) {
         double su = 0.0;
         for (int c = 0; c < DM; ++c) su = su + sh[c][0];
@@ -829,12 +844,17 @@ void launch_maxpy_norm(const Dims& D, double* w, const MVecs& V, int J, const do
                        unsigned* counter, double* out, cudaStream_t s, int ninst, int64_t ss) {
     const int64_t n = (int64_t)D.nx * D.ny * (D.dm == 3 ? D.nz : 1);
     const int vec = pairs_ok(D, w, V, J);
-    const int cl = cgs_cluster(n);
+    const int cl = cgs_cluster(n), nc = D.dm + 1;
+    const bool cs = cl ? cl * nc <= 8 : mdot_blocks(n) * ninst <= 148;   // split by component (k_reduce)
 #define MN(DM_, J_)                                                                                                     \
-    if (cl)                                                                                                             \
-        launch_cluster(k_maxpy_norm<DM_, J_, true>, dim3(cl, ninst), dim3(kMdotThreads), cl, 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec); \
+    if (cl && cs)                                                                                                       \
+        launch_cluster(k_maxpy_norm<DM_, J_, true, true>, dim3(cl, ninst, nc), dim3(kMdotThreads), dim3(cl, 1, nc), 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec); \
+    else if (cl)                                                                                                        \
+        launch_cluster(k_maxpy_norm<DM_, J_, true, false>, dim3(cl, ninst), dim3(kMdotThreads), dim3(cl), 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec); \
+    else if (cs)                                                                                                        \
+        launch_pdl(k_maxpy_norm<DM_, J_, false, true>, dim3(mdot_blocks(n), ninst, nc), dim3(kMdotThreads), 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec); \
     else                                                                                                                \
-        launch_pdl(k_maxpy_norm<DM_, J_, false>, dim3(cgs_blocks<DM_, J_, true>(n), ninst), dim3(kMdotThreads), 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec)
+        launch_pdl(k_maxpy_norm<DM_, J_, false, false>, dim3(cgs_blocks<DM_, J_, true>(n), ninst), dim3(kMdotThreads), 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec)
 #define MNJ(DM_)                               \
     switch (J) {                               \
     case 1: MN(DM_, 1); break;                 \
@@ -867,7 +887,7 @@ int cgs_blocks(int64_t n) {
         int dev = 0, sms = 148, per_sm = 4;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const void* k = NORM ? (const void*)k_maxpy_norm<DM, J, false> : (const void*)k_mdot<DM, J, false>;
+        const void* k = NORM ? (const void*)k_maxpy_norm<DM, J, false, false> : (const void*)k_mdot<DM, J, false, false>;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kMdotThreads, 0) != cudaSuccess || per_sm < 1) {
             cudaGetLastError();
             per_sm = 1;
@@ -882,12 +902,17 @@ void launch_mdot(const Dims& D, const double* w, const MVecs& V, int J, double w
                  double* out, cudaStream_t s, int ninst, int64_t ss) {
     const int64_t n = (int64_t)D.nx * D.ny * (D.dm == 3 ? D.nz : 1);
     const int vec = pairs_ok(D, w, V, J);
-    const int cl = cgs_cluster(n);
+    const int cl = cgs_cluster(n), nc = D.dm + 1;
+    const bool cs = cl ? cl * nc <= 8 : mdot_blocks(n) * ninst <= 148;   // split by component (k_reduce)
 #define MD(DM_, J_)                                                                                                     \
-    if (cl)                                                                                                             \
-        launch_cluster(k_mdot<DM_, J_, true>, dim3(cl, ninst), dim3(kMdotThreads), cl, 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec); \
+    if (cl && cs)                                                                                                       \
+        launch_cluster(k_mdot<DM_, J_, true, true>, dim3(cl, ninst, nc), dim3(kMdotThreads), dim3(cl, 1, nc), 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec); \
+    else if (cl)                                                                                                        \
+        launch_cluster(k_mdot<DM_, J_, true, false>, dim3(cl, ninst), dim3(kMdotThreads), dim3(cl), 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec); \
+    else if (cs)                                                                                                        \
+        launch_pdl(k_mdot<DM_, J_, false, true>, dim3(mdot_blocks(n), ninst, nc), dim3(kMdotThreads), 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec); \
     else                                                                                                                \
-        launch_pdl(k_mdot<DM_, J_, false>, dim3(cgs_blocks<DM_, J_, false>(n), ninst), dim3(kMdotThreads), 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec)
+        launch_pdl(k_mdot<DM_, J_, false, false>, dim3(cgs_blocks<DM_, J_, false>(n), ninst), dim3(kMdotThreads), 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec)
 #define MDJ(DM_)                               \
     switch (J) {                               \
     case 1: MD(DM_, 1); break;                 \

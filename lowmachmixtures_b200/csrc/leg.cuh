@@ -328,7 +328,7 @@ static cudaError_t launch_leg_k(K kernel, const A& args, const LegShape& sh, int
         e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
-    return launch_cluster(kernel, dim3(blocks * sh.nc), dim3(sh.threads), sh.nc, sh.smem, s, args);
+    return launch_cluster(kernel, dim3(blocks * sh.nc), dim3(sh.threads), dim3(sh.nc), sh.smem, s, args);
 }
 
 template <class T, int DM, bool W, int PP>
