@@ -258,79 +258,95 @@ void launch_add_scaled_multi_f32(double* x, const MZ32& Z, const YS& ys, int J, 
 }
 
 // ---------------------------------------------------------------- Schur complement pieces
+// kSchurPer entries per thread, a block apart: one was bound by the loads in flight (256^3 FP32, theta = 0: 74 us for 201 MB; 31 now, the rate of a copy)
+constexpr int kSchurPer = 4;
 template <class T>
 __global__ void k_schur(int mode, int pt, int av, double theta, const T* __restrict__ mac, const T* __restrict__ src,
                         const T* __restrict__ beta, const T* __restrict__ gamma, T* __restrict__ phi, const T* __restrict__ bp,
                         T* __restrict__ xp, int64_t n) {
     pdl_enter();
-    int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= n) return;
     const T th = (T)theta;
-    T x = 0;
-    if (mode == 0) {  // simple_schur_complement (apply_precon.f90:485-528) [+ sign flip :244-249]
-        if (av == 1 || av == 2) {
-            x = mac[t] * T(-1);
-            x = x * beta[t];
-            if (av == 2) x = x * T(2);
-        } else {
-            x = mac[t] * T(-4.0 / 3.0);
-            x = x * beta[t];
-            T m2 = mac[t] * T(-1);
-            m2 = m2 * gamma[t];
-            x = x + m2;
-        }
-        if (fabs(theta) > 0.0) {
-            T ph = phi[t] * th;
+    const int64_t t0 = (int64_t)blockIdx.x * (kT * kSchurPer) + threadIdx.x;
+    const bool with_mac = mode == 0 || (mode == 1 && (pt == 1 || theta == 0.0)), with_phi = mode != 0 || fabs(theta) > 0.0;
+    T ma[kSchurPer], be[kSchurPer], pv[kSchurPer];
+#pragma unroll
+    for (int e = 0; e < kSchurPer; ++e) {
+        const int64_t t = t0 + e * kT;
+        const bool in = t < n;
+        ma[e] = in && with_mac ? mac[t] : T(0);
+        be[e] = in ? beta[t] : T(0);
+        pv[e] = in && with_phi ? phi[t] : T(0);
+    }
+#pragma unroll
+    for (int e = 0; e < kSchurPer; ++e) {
+        const int64_t t = t0 + e * kT;
+        if (t >= n) return;
+        T x = 0;
+        if (mode == 0) {  // simple_schur_complement (apply_precon.f90:485-528) [+ sign flip :244-249]
+            if (av == 1 || av == 2) {
+                x = ma[e] * T(-1);
+                x = x * be[e];
+                if (av == 2) x = x * T(2);
+            } else {
+                x = ma[e] * T(-4.0 / 3.0);
+                x = x * be[e];
+                T m2 = ma[e] * T(-1);
+                m2 = m2 * gamma[t];
+                x = x + m2;
+            }
+            if (fabs(theta) > 0.0) {
+                T ph = pv[e] * th;
+                phi[t] = ph;
+                x = x + ph;
+            }
+            if (pt == -2 || pt == -5) x = x * T(-1);
+        } else if (mode == 1) {  // projection preconditioner (apply_precon.f90:140-188)
+            T sv = (pt == 1 || theta == 0.0) ? ma[e] * T(-1) : src[t];
+            if (av == 1 || av == 2) {
+                x = sv * be[e];
+                if (av == 2) x = x * T(2);
+            } else {
+                T m2 = sv * gamma[t];
+                x = sv * be[e];
+                x = x * T(4.0 / 3.0);
+                x = x + m2;
+            }
+            T ph = pv[e] * th;
             phi[t] = ph;
             x = x + ph;
+        } else {  // block diagonal (apply_precon.f90:380-416)
+            T ph = pv[e];
+            if (fabs(theta) > 0.0) {
+                ph = ph * th;
+                phi[t] = ph;
+            }
+            x = bp[t] * be[e];
+            x = x - ph;
+            if (av == 1 && pt == 4) {
+                x = x * T(-1);
+            } else if (av == 2 && pt == 4) {
+                x = x * T(-2);
+            } else if (av == 2 && pt == -4) {
+                x = x * T(2);
+            } else if (av == 3 && pt == 4) {
+                x = x * T(-4.0 / 3.0);
+                T q = bp[t] * gamma[t];
+                q = q * T(-1);
+                x = x + q;
+            } else if (av == 3 && pt == -4) {
+                x = x * T(4.0 / 3.0);
+                T q = bp[t] * gamma[t];
+                x = x + q;
+            }
         }
-        if (pt == -2 || pt == -5) x = x * T(-1);
-    } else if (mode == 1) {  // projection preconditioner (apply_precon.f90:140-188)
-        T sv = (pt == 1 || theta == 0.0) ? mac[t] * T(-1) : src[t];
-        if (av == 1 || av == 2) {
-            x = sv * beta[t];
-            if (av == 2) x = x * T(2);
-        } else {
-            T m2 = sv * gamma[t];
-            x = sv * beta[t];
-            x = x * T(4.0 / 3.0);
-            x = x + m2;
-        }
-        T ph = phi[t] * th;
-        phi[t] = ph;
-        x = x + ph;
-    } else {  // block diagonal (apply_precon.f90:380-416)
-        T ph = phi[t];
-        if (fabs(theta) > 0.0) {
-            ph = ph * th;
-            phi[t] = ph;
-        }
-        x = bp[t] * beta[t];
-        x = x - ph;
-        if (av == 1 && pt == 4) {
-            x = x * T(-1);
-        } else if (av == 2 && pt == 4) {
-            x = x * T(-2);
-        } else if (av == 2 && pt == -4) {
-            x = x * T(2);
-        } else if (av == 3 && pt == 4) {
-            x = x * T(-4.0 / 3.0);
-            T q = bp[t] * gamma[t];
-            q = q * T(-1);
-            x = x + q;
-        } else if (av == 3 && pt == -4) {
-            x = x * T(4.0 / 3.0);
-            T q = bp[t] * gamma[t];
-            x = x + q;
-        }
+        xp[t] = x;
     }
-    xp[t] = x;
 }
 
 template <class T>
 void launch_schur(int mode, int precon_type, int visc_abs, double theta_alpha, const T* mac_rhs, const T* src,
                   const T* beta, const T* gamma, T* phi, const T* bp, T* xp, int64_t n, cudaStream_t s) {
-    launch_pdl(k_schur<T>, nb(n), kT, 0, s, mode, precon_type, visc_abs, theta_alpha, mac_rhs, src, beta, gamma, phi, bp, xp, n);
+    launch_pdl(k_schur<T>, dim3((unsigned)((n + kT * kSchurPer - 1) / (kT * kSchurPer))), dim3(kT), 0, s, mode, precon_type, visc_abs, theta_alpha, mac_rhs, src, beta, gamma, phi, bp, xp, n);
 }
 template void launch_schur<double>(int, int, int, double, const double*, const double*, const double*, const double*, double*,
                                    const double*, double*, int64_t, cudaStream_t);
@@ -338,35 +354,45 @@ template void launch_schur<float>(int, int, int, double, const float*, const flo
                                   const float*, float*, int64_t, cudaStream_t);
 
 // ---------------------------------------------------------------- mean removal
-// sub_u: bit d set = remove the mean of velocity component d
+// sub_u: bit d set = remove the mean of velocity component d.  A block takes
+// kSubPer entries per thread, a block apart, and forms the means once (they
+// were four FP64 divisions per entry: 180 us at 256^3 FP32 against 82 of traffic;
+// 85 now).
+constexpr int kSubPer = 4;
 template <class T, int DM>
-__global__ void k_sub_means(Dims D, T* u0, T* u1, T* u2, T* p, const double* __restrict__ sums, double total_volume, int sub_u) {
+__global__ void __launch_bounds__(kT) k_sub_means(Dims D, T* __restrict__ u0, T* __restrict__ u1, T* __restrict__ u2, T* __restrict__ p,
+                                                  const double* __restrict__ sums, double total_volume, int sub_u) {
     pdl_enter();
-    int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    int64_t n = (int64_t)D.nx * D.ny * D.nz;
-    if (t >= n) return;
-    // 2D batch: the sums of this entry's instance (slot stride 8)
-    if (DM == 2) sums += (int64_t)((int)t / (D.nx * D.ny)) * 8;
-    const double mp = sums[DM] / total_volume;
-    p[t] = (T)((double)p[t] - mp);
-    if (sub_u) {
-        T* u[3] = {u0, u1, u2};
+    // 2D batch: blockIdx.y is the instance, its sums (slot stride 8)
+    const int64_t ni = (int64_t)D.nx * D.ny * (DM == 3 ? D.nz : 1), off = ni * blockIdx.y;
+    sums += (int64_t)blockIdx.y * 8;
+    __shared__ double mean[DM + 1];
+    if (threadIdx.x <= DM) mean[threadIdx.x] = sums[threadIdx.x] / total_volume;
+    __syncthreads();
+    const int64_t t0 = (int64_t)blockIdx.x * (kT * kSubPer) + threadIdx.x;
 #pragma unroll
-        for (int d = 0; d < DM; ++d) {
-            if (!((sub_u >> d) & 1)) continue;
-            const double mu = sums[d] / total_volume;
-            u[d][t] = (T)((double)u[d][t] - mu);
-        }
+    for (int d = 0; d <= DM; ++d) {
+        if (d < DM && !((sub_u >> d) & 1)) continue;
+        T* x = (d == DM ? p : (d == 0 ? u0 : (d == 1 ? u1 : u2))) + off;
+        const double m = mean[d];
+        T v[kSubPer];
+#pragma unroll
+        for (int q = 0; q < kSubPer; ++q)
+            if (t0 + q * kT < ni) v[q] = x[t0 + q * kT];
+#pragma unroll
+        for (int q = 0; q < kSubPer; ++q)
+            if (t0 + q * kT < ni) x[t0 + q * kT] = (T)((double)v[q] - m);
     }
 }
 
 template <class T>
 void launch_sub_means(const Dims& D, T* const u[3], T* p, const double* sums, double total_volume, int sub_u, cudaStream_t s) {
-    int64_t n = (int64_t)D.nx * D.ny * D.nz;
+    const int64_t ni = (int64_t)D.nx * D.ny * (D.dm == 3 ? D.nz : 1);
+    const dim3 g((unsigned)((ni + kT * kSubPer - 1) / (kT * kSubPer)), D.dm == 2 ? D.nz : 1);
     if (D.dm == 2)
-        launch_pdl(k_sub_means<T, 2>, nb(n), kT, 0, s, D, u[0], u[1], u[2], p, sums, total_volume, sub_u);
+        launch_pdl(k_sub_means<T, 2>, g, dim3(kT), 0, s, D, u[0], u[1], u[2], p, sums, total_volume, sub_u);
     else
-        launch_pdl(k_sub_means<T, 3>, nb(n), kT, 0, s, D, u[0], u[1], u[2], p, sums, total_volume, sub_u);
+        launch_pdl(k_sub_means<T, 3>, g, dim3(kT), 0, s, D, u[0], u[1], u[2], p, sums, total_volume, sub_u);
 }
 template void launch_sub_means<double>(const Dims&, double* const[3], double*, const double*, double, int, cudaStream_t);
 template void launch_sub_means<float>(const Dims&, float* const[3], float*, const double*, double, int, cudaStream_t);
