@@ -980,49 +980,82 @@ void launch_maxpy(double* w, const MVecs& V, int J, const double* hs, int64_t le
 // above with that instance's scalar.
 namespace {
 
-__device__ __forceinline__ int inst_of(int64_t e, int64_t n, int ni) { return (int)((e % n) / ni); }
+// The pointwise batch kernels: blockIdx.y is the instance, blockIdx.z the
+// component, a thread takes kBatchPer entries a block apart.  With the instance
+// worked out per entry (a 64-bit modulo and division) they were bound by that:
+// k_div_by_batch 7.5 us on average over an ensemble of 96 problems, 4.3 now.
+constexpr int kBatchPer = 4;
+struct BatchPos {
+    int64_t base;   // of the instance's component
+    int t0;
+};
+__device__ __forceinline__ BatchPos batch_pos(int64_t n, int ni) {
+    return {(int64_t)blockIdx.z * n + (int64_t)blockIdx.y * ni, (int)(blockIdx.x * (kT * kBatchPer) + threadIdx.x)};
+}
+static dim3 batch_grid(int64_t n, int ni, int64_t len) {
+    return dim3((unsigned)((ni + kT * kBatchPer - 1) / (kT * kBatchPer)), (unsigned)(n / ni), (unsigned)(len / n));
+}
 
 // v = w / den_b (den_b = slots[8b + 5]); v32 (may be null) = (float)v.  A
 // zero norm (an instance that has stopped: its column is not used) divides
 // by 1 instead.
 __global__ void k_div_by_batch(const double* __restrict__ w, double* __restrict__ v, float* __restrict__ v32,
-                               const double* __restrict__ slots, int64_t n, int ni, int64_t len) {
+                               const double* __restrict__ slots, int64_t n, int ni) {
     pdl_enter();
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= len) return;
-    const double d = slots[(int64_t)inst_of(e, n, ni) * 8 + 5];
-    const double q = w[e] / (d != 0.0 ? d : 1.0);
-    v[e] = q;
-    if (v32) v32[e] = (float)q;
+    const BatchPos p = batch_pos(n, ni);
+    const double s = slots[(int64_t)blockIdx.y * 8 + 5], d = s != 0.0 ? s : 1.0;
+    double x[kBatchPer];
+#pragma unroll
+    for (int q = 0; q < kBatchPer; ++q) x[q] = p.t0 + q * kT < ni ? w[p.base + p.t0 + q * kT] : 0.0;
+#pragma unroll
+    for (int q = 0; q < kBatchPer; ++q) {
+        if (p.t0 + q * kT >= ni) return;
+        const int64_t e = p.base + p.t0 + q * kT;
+        const double y = x[q] / d;
+        v[e] = y;
+        if (v32) v32[e] = (float)y;
+    }
 }
 
 // w -= V * h_b (h_b = slots[8b + 4])
 __global__ void k_sub_scaled_batch(double* __restrict__ w, const double* __restrict__ V, const double* __restrict__ slots, int64_t n,
-                                   int ni, int64_t len) {
+                                   int ni) {
     pdl_enter();
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= len) return;
-    const double tmp = V[e] * slots[(int64_t)inst_of(e, n, ni) * 8 + 4];
-    w[e] = w[e] - tmp;
+    const BatchPos p = batch_pos(n, ni);
+    const double h = slots[(int64_t)blockIdx.y * 8 + 4];
+#pragma unroll
+    for (int q = 0; q < kBatchPer; ++q) {
+        if (p.t0 + q * kT >= ni) return;
+        const int64_t e = p.base + p.t0 + q * kT;
+        const double tmp = V[e] * h;
+        w[e] = w[e] - tmp;
+    }
 }
 
 // x += sum_{k<J} ys[k*B + b] Z_k, in k order; a zero coefficient (an
 // instance whose cycle had fewer columns) is skipped
 template <class TZ>
 __global__ void k_add_scaled_multi_batch(double* __restrict__ x, const TZ* const* __restrict__ Z, const double* __restrict__ ys, int J,
-                                         int nbatch, int64_t n, int ni, int64_t len) {
+                                         int nbatch, int64_t n, int ni) {
     pdl_enter();
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < len; e += (int64_t)gridDim.x * blockDim.x) {
-        const int b = inst_of(e, n, ni);
-        double v = x[e];
-        for (int k = 0; k < J; ++k) {
-            const double y = ys[(int64_t)k * nbatch + b];
-            if (y == 0.0) continue;
-            const double tmp = (double)Z[k][e] * y;
-            v = v + tmp;
-        }
-        x[e] = v;
+    const BatchPos p = batch_pos(n, ni);
+    double v[kBatchPer];
+#pragma unroll
+    for (int q = 0; q < kBatchPer; ++q) v[q] = p.t0 + q * kT < ni ? x[p.base + p.t0 + q * kT] : 0.0;
+    for (int k = 0; k < J; ++k) {
+        const double y = ys[(int64_t)k * nbatch + blockIdx.y];
+        if (y == 0.0) continue;
+        const TZ* z = Z[k] + p.base;
+#pragma unroll
+        for (int q = 0; q < kBatchPer; ++q)
+            if (p.t0 + q * kT < ni) {
+                const double tmp = (double)z[p.t0 + q * kT] * y;
+                v[q] = v[q] + tmp;
+            }
     }
+#pragma unroll
+    for (int q = 0; q < kBatchPer; ++q)
+        if (p.t0 + q * kT < ni) x[p.base + p.t0 + q * kT] = v[q];
 }
 
 // dst[b * ni + t] = src[b][t] and back (per-instance arrays <-> batch array)
@@ -1042,17 +1075,15 @@ __global__ void k_scatter_ptrs(const double* __restrict__ src, double* const* __
 }  // namespace
 
 void launch_div_by_batch(const double* w, double* v, float* v32, const double* slots, int64_t n, int ni, int64_t len, cudaStream_t s) {
-    launch_pdl(k_div_by_batch, nb(len), kT, 0, s, w, v, v32, slots, n, ni, len);
+    launch_pdl(k_div_by_batch, batch_grid(n, ni, len), dim3(kT), 0, s, w, v, v32, slots, n, ni);
 }
 void launch_sub_scaled_batch(double* w, const double* V, const double* slots, int64_t n, int ni, int64_t len, cudaStream_t s) {
-    launch_pdl(k_sub_scaled_batch, nb(len), kT, 0, s, w, V, slots, n, ni, len);
+    launch_pdl(k_sub_scaled_batch, batch_grid(n, ni, len), dim3(kT), 0, s, w, V, slots, n, ni);
 }
 template <class TZ>
 void launch_add_scaled_multi_batch(double* x, const TZ* const* Z_dev, const double* ys_dev, int J, int nbatch, int64_t n, int ni,
                                    int64_t len, cudaStream_t s) {
-    const int64_t b = (len + kT - 1) / kT;
-    const int g = (int)(b > 8192 ? 8192 : b);
-    launch_pdl(k_add_scaled_multi_batch<TZ>, g, kT, 0, s, x, Z_dev, ys_dev, J, nbatch, n, ni, len);
+    launch_pdl(k_add_scaled_multi_batch<TZ>, batch_grid(n, ni, len), dim3(kT), 0, s, x, Z_dev, ys_dev, J, nbatch, n, ni);
 }
 template void launch_add_scaled_multi_batch<float>(double*, const float* const*, const double*, int, int, int64_t, int, int64_t,
                                                    cudaStream_t);
