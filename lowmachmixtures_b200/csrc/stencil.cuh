@@ -55,17 +55,19 @@ static __device__ bc::Table g_bc_table;
 static __device__ bc::Record g_bc_record;
 // a load of `bytes` at p: in shared memory it must lie within this CTA's
 // shared memory (static + dynamic), in global memory within a registered
-// allocation; other windows (local) are not tracked
-__device__ __forceinline__ bool bc_ok(const void* p, unsigned bytes) {
+// allocation; other windows (local) are not tracked.  A call, not inlined: it
+// sits behind every load, and inlined it is most of this build's compile time.
+static __device__ __noinline__ bool bc_ok(const void* p, unsigned bytes) {
     const unsigned long long a = reinterpret_cast<unsigned long long>(p);
     bool ok;
     if (__isShared(p)) {
         // the CTA's own shared memory (static, then dynamic) follows the
-        // reserved region: offsets [cap, cap + total)
+        // reserved region: offsets [cap, cap + total).  In a cluster the window
+        // holds every CTA's, 16 MB apart: the offset is the low 24 bits
         unsigned total, cap;
         asm("mov.u32 %0, %%total_smem_size;" : "=r"(total));
         asm("mov.u32 %0, %%reserved_smem_offset_cap;" : "=r"(cap));
-        const unsigned long long off = __cvta_generic_to_shared(p);
+        const unsigned long long off = __cvta_generic_to_shared(p) & 0xffffffull;
         ok = off >= cap && off + bytes <= (unsigned long long)cap + total;
     } else if (__isGlobal(p)) {
         ok = false;
