@@ -238,7 +238,11 @@ int lmm_stokes_create(const lmm_grid* g, const lmm_knobs* k, int device, lmm_han
 int lmm_stokes_solve(lmm_handle* h, const lmm_fields_in* in, lmm_fields_out* out,
                      double* theta_alpha, double* norm_pre_rhs, lmm_stats* st);
 
-/* Same solve on device-resident LMM_LAYOUT_COMPACT arrays (no host copies). */
+/* Same solve on device-resident LMM_LAYOUT_COMPACT arrays (no host copies).
+ * Arrays in memory of the handle's device are read and written in place; any
+ * other that cudaMemcpyAsync takes (pinned or managed memory, another device's,
+ * one not on an 8-byte boundary) is copied, and one that it does not know is
+ * LMM_ERR_CUDA.  The same holds for lmm_op_load_coeffs and lmm_op_apply_matrix. */
 int lmm_stokes_solve_device(lmm_handle* h, const lmm_fields_in* in_dev, lmm_fields_out* out_dev,
                             double* theta_alpha, double* norm_pre_rhs, lmm_stats* st);
 

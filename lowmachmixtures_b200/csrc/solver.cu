@@ -13,6 +13,7 @@
 // Scalars of the Arnoldi process (H, norms) stay on the device; the host
 // reads one Hessenberg column per inner iteration to run the Givens
 // rotations and the stopping tests exactly as the reference does.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -593,6 +594,85 @@ double read_slot(lmm_handle* h, int slot, int idx) {
     return h->hscal[idx];
 }
 
+// ------------------------------------------------------------ the caller's arrays
+// Which of an entry point's arrays its kernels may read and write in place:
+// device memory of the handle's device and of the current context, the whole
+// array in one allocation, on an 8-byte boundary.  Any other one is copied
+// (cudaMemcpyAsync) to or from the handle's buffers: a copy takes pinned and
+// managed memory and another GPU's without peer access, and reports an address
+// it does not know as an error; a kernel would fault on it.  One object per
+// call: what it learns about an allocation holds for that call only.
+class CallerArrays {
+public:
+    explicit CallerArrays(const lmm_handle* h) : device_(h->device) {}
+    bool in_place(const void* p, size_t bytes) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+        if (!p || a % sizeof(double) != 0) return false;
+        if (a >= lo_ && a < hi_ && bytes <= hi_ - a) return true;   // the last array's allocation
+        // the driver's query, fetched through the runtime (the library does not link libcuda); it
+        // takes any address, and leaves zeros for one that it does not know
+        static const auto query = entry<decltype(&cuPointerGetAttributes)>("cuPointerGetAttributes");
+        static const auto current = entry<decltype(&cuCtxGetCurrent)>("cuCtxGetCurrent");
+        unsigned type = 0, managed = 0;
+        int device = -1;
+        CUdeviceptr base = 0;
+        size_t size = 0;
+        CUcontext owner = nullptr, ctx = nullptr;   // owner null: memory of a pool, of no one context
+        CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                      CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,   CU_POINTER_ATTRIBUTE_CONTEXT,
+                                      CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+        void* out[] = {&type, &managed, &device, &owner, &base, &size};
+        if (!query || !current || query(6, what, out, (CUdeviceptr)a) != CUDA_SUCCESS || current(&ctx) != CUDA_SUCCESS) return false;
+        if (type != CU_MEMORYTYPE_DEVICE || managed || device != device_ || (owner && owner != ctx)) return false;
+        if (a < base || a - base > size || bytes > size - (a - base)) return false;
+        lo_ = base;
+        hi_ = base + size;
+        return true;
+    }
+
+private:
+    template <class F>
+    static F entry(const char* name) {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return reinterpret_cast<F>(p);
+    }
+    int device_;
+    uintptr_t lo_ = 0, hi_ = 0;
+};
+// the copy an array that is not used in place takes
+void copy_array(lmm_handle* h, double* dst, const double* src, int64_t count) {
+    if (!dst || !src) {
+        note_error("a required array is missing", __func__, __LINE__);
+        throw LmmError(LMM_ERR_CUDA);
+    }
+    LMM_CK(cudaMemcpyAsync(dst, src, count * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+}
+// dst <- src for up to 8 fields, at least one side of each the handle's: those
+// in place in one launch, the others by copies
+struct FieldCopies {
+    lmm_handle* h;
+    CallerArrays arrays;
+    CopyFields A{};
+    int count = 0;
+    explicit FieldCopies(lmm_handle* handle) : h(handle), arrays(handle) { A.n = handle->n; }
+    // caller: the side that is the caller's
+    void add(double* dst, const double* src, const double* caller) {
+        if (!arrays.in_place(caller, h->n * sizeof(double))) return copy_array(h, dst, src, h->n);
+        A.src[count] = src;
+        A.dst[count++] = dst;
+    }
+    void run() {
+        if (count == 0) return;
+        launch_copy_fields(A, count, h->stream);
+        check_launch();
+    }
+};
+
 // ------------------------------------------------------------ coefficients
 // Level-0 coefficients in FP64 (theta*alpha, beta, beta_ed, gamma), the
 // hierarchy by coarsening (stag_mg_solver.f90:200-230, hoisted out of the
@@ -602,6 +682,13 @@ void load_coeffs(lmm_handle* h, const double* const alpha_dev[3], const double* 
     const int dm = h->dm, nedge = dm == 2 ? 1 : 3;
     const bool fp32 = h->knobs.precision == LMM_PRECISION_FP32;
     LevelDev<double>& L0 = h->L64[0];
+    // an array the kernels cannot read where it is goes to the level's own first
+    CallerArrays arrays(h);
+    auto at = [&](const double* src, double* own, int64_t count) -> const double* {
+        if (src == own || arrays.in_place(src, count * sizeof(double))) return src;
+        copy_array(h, own, src, count);
+        return own;
+    };
     // flags and values of the uniform levels (see below): 32 values, 32 flags
     double* vals = h->ustate;
     int* flags = reinterpret_cast<int*>(h->ustate + 32);
@@ -618,19 +705,19 @@ void load_coeffs(lmm_handle* h, const double* const alpha_dev[3], const double* 
         CoefFine A{};
         A.D = L0.D;
         A.theta = theta;
-        A.beta = beta;
-        A.gamma = gamma;
+        A.beta = at(beta, L0.beta, h->n);
+        A.gamma = gamma ? at(gamma, L0.gamma, h->n) : nullptr;
         A.o_beta = L0.beta;
         A.o_gamma = L0.gamma;
         for (int d = 0; d < dm; ++d) {
-            A.alpha[d] = alpha_dev[d];
+            A.alpha[d] = at(alpha_dev[d], h->alpha_fc[d], h->n);
             A.o_alpha[d] = L0.alpha[d];
             A.o_ainv[d] = h->alphainv[d];
             if (h->D0.wall && h->nlev_p > 0) A.o_pa[d] = L0.pa[d];
         }
         for (int e = 0; e < nedge; ++e) {
-            A.bed[e] = bed[e];
             A.ne[e] = edge_count(L0.D, e);
+            A.bed[e] = at(bed[e], L0.bed[e], A.ne[e]);
             A.o_bed[e] = L0.bed[e];
         }
         if (fp32) {
@@ -2666,31 +2753,24 @@ int solve_core(lmm_handle* h, const lmm_fields_in* in, const double* x0_u[3], co
     LevelDev<double>& L0 = h->L64[0];
     // b = (scaled) rhs, x = (scaled) initial guess
     {
-        CopyFields A{};
-        A.n = n;
-        int q = 0;
-        auto copy = [&](const double* src, double* dst) {
-            A.src[q] = src;
-            A.dst[q++] = dst;
-        };
+        FieldCopies f(h);
         for (int d = 0; d < dm; ++d) {
             if (sf != 1.0) {
                 launch_scale_copy<double>(in->b_u[d], h->b.c(d), sf, n, h->stream);
                 check_launch();
             } else {
-                copy(in->b_u[d], h->b.c(d));
+                f.add(h->b.c(d), in->b_u[d], in->b_u[d]);
             }
-            copy(x0_u[d], h->x.c(d));
+            f.add(h->x.c(d), x0_u[d], x0_u[d]);
         }
-        copy(in->b_p, h->b.p());
+        f.add(h->b.p(), in->b_p, in->b_p);
         if (sf != 1.0) {
             launch_scale_copy<double>(x0_p, h->x.p(), sf, n, h->stream);
             check_launch();
         } else {
-            copy(x0_p, h->x.p());
+            f.add(h->x.p(), x0_p, x0_p);
         }
-        launch_copy_fields(A, q, h->stream);
-        check_launch();
+        f.run();
     }
     if (h->D0.wall) {
         // wall-normal velocities on the walls are not unknowns: zero in x
@@ -2765,16 +2845,10 @@ extern "C" int lmm_stokes_solve_device(lmm_handle* h, const lmm_fields_in* in, l
         const double* x0u[3] = {out->x_u[0], out->x_u[1], out->x_u[2]};
         int rc = solve_core(h, in, x0u, out->x_p, theta_alpha, norm_pre_rhs, st);
         if (rc >= 0 || rc == LMM_ERR_BREAKDOWN || rc == LMM_ERR_NONFINITE) {
-            CopyFields A{};
-            A.n = h->n;
-            for (int d = 0; d < h->dm; ++d) {
-                A.src[d] = h->x.c(d);
-                A.dst[d] = out->x_u[d];
-            }
-            A.src[h->dm] = h->x.p();
-            A.dst[h->dm] = out->x_p;
-            launch_copy_fields(A, h->dm + 1, h->stream);
-            check_launch();
+            FieldCopies f(h);
+            for (int d = 0; d < h->dm; ++d) f.add(out->x_u[d], h->x.c(d), out->x_u[d]);
+            f.add(out->x_p, h->x.p(), out->x_p);
+            f.run();
         }
         LMM_CK(cudaEventRecord(h->ev1, h->stream));
         LMM_CK(host_wait(h));
@@ -3094,9 +3168,10 @@ extern "C" int lmm_op_apply_matrix(lmm_handle* h, const double* const x_u[3], co
     try {
         const int dm = h->dm;
         const int64_t n = h->n;
-        // the caller's arrays in place, unless an output overlaps an input or
-        // another output (then through the handle's vectors)
+        // the caller's arrays in place, unless one of them cannot be (CallerArrays)
+        // or an output overlaps an input or another output (then through the handle's vectors)
         {
+            CallerArrays arrays(h);
             const double* x[4] = {x_u[0], x_u[1], dm == 3 ? x_u[2] : x_u[0], x_p};
             double* b[4] = {b_u[0], b_u[1], dm == 3 ? b_u[2] : b_u[0], b_p};
             auto apart = [&](const double* p, const double* q) {
@@ -3106,6 +3181,7 @@ extern "C" int lmm_op_apply_matrix(lmm_handle* h, const double* const x_u[3], co
             bool ok = true;
             for (int i = 0; i < 4; ++i) {
                 if (dm == 2 && i == 2) continue;
+                ok = ok && arrays.in_place(x[i], n * sizeof(double)) && arrays.in_place(b[i], n * sizeof(double));
                 for (int j = 0; j < 4; ++j) {
                     if (dm == 2 && j == 2) continue;
                     ok = ok && apart(b[i], x[j]) && (i == j || apart(b[i], b[j]));
@@ -3119,14 +3195,12 @@ extern "C" int lmm_op_apply_matrix(lmm_handle* h, const double* const x_u[3], co
                 return bc_status();
             }
         }
-        for (int d = 0; d < dm; ++d)
-            LMM_CK(cudaMemcpyAsync(h->r.c(d), x_u[d], n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-        LMM_CK(cudaMemcpyAsync(h->r.p(), x_p, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+        for (int d = 0; d < dm; ++d) copy_array(h, h->r.c(d), x_u[d], n);
+        copy_array(h, h->r.p(), x_p, n);
         launch_apply_matrix(h->L64[0], h->knobs.visc_type, h->r, h->tmp, h->stream);
         check_launch();
-        for (int d = 0; d < dm; ++d)
-            LMM_CK(cudaMemcpyAsync(b_u[d], h->tmp.c(d), n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-        LMM_CK(cudaMemcpyAsync(b_p, h->tmp.p(), n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+        for (int d = 0; d < dm; ++d) copy_array(h, b_u[d], h->tmp.c(d), n);
+        copy_array(h, b_p, h->tmp.p(), n);
         LMM_CK(host_wait(h));
         return bc_status();
     } catch (const LmmError& e) {
