@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "stencil.cuh"
+
 namespace lmm {
 
 // every thread of every block arrives; the two halves of cluster_sync.  A block
@@ -32,8 +34,18 @@ __device__ __forceinline__ unsigned dsmem_at(unsigned a, unsigned r) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(r));
     return o;
 }
-__device__ __forceinline__ void dsmem_store(unsigned a, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
-__device__ __forceinline__ void dsmem_store(unsigned a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
+__device__ __forceinline__ void dsmem_store(unsigned a, float v) {
+#ifdef LMM_BOUNDS_CHECK
+    if (!bc_cluster_ok(a, sizeof(v))) return;
+#endif
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void dsmem_store(unsigned a, double v) {
+#ifdef LMM_BOUNDS_CHECK
+    if (!bc_cluster_ok(a, sizeof(v))) return;
+#endif
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
 
 // clusters of nc.x x nc.y x nc.z blocks, ranked x fastest (each extent of the grid a multiple of its)
 template <class... KArgs, class... Args>

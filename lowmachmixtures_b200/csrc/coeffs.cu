@@ -23,6 +23,10 @@ inline int blocks(int64_t n) { return (int)std::max<int64_t>(1, (n + kT - 1) / k
 
 __device__ __forceinline__ bool differs(double a, double b) { return __double_as_longlong(a) != __double_as_longlong(b); }
 
+// entry t of an array of the finest level, which may be the output array
+// itself (a plain load); a field holds fewer than 2^31 entries
+__device__ __forceinline__ double in(const double* p, int64_t t) { return ldp<1>(p, (int)t); }
+
 // flags of a block: set where a thread saw a value that differs
 __device__ __forceinline__ void raise(bool diff, int* flag) {
     if (__syncthreads_or(diff) && threadIdx.x == 0) *flag = 1;
@@ -41,7 +45,7 @@ __global__ void __launch_bounds__(kT) k_coeffs_fine(CoefFine A) {
     pdl_enter();
     const int64_t t = blockIdx.x * (int64_t)kT + threadIdx.x;
     const int64_t n = (int64_t)A.D.nx * A.D.ny * A.D.nz;
-    const double a0 = A.alpha[0][0], s0 = a0 * A.theta, r0 = 1.0 / a0;
+    const double a0 = in(A.alpha[0], 0), s0 = a0 * A.theta, r0 = 1.0 / a0;
     bool ds = false, dr = false;
     if (t < n) {
         int x[3] = {1, 1, 1};
@@ -53,7 +57,7 @@ __global__ void __launch_bounds__(kT) k_coeffs_fine(CoefFine A) {
         }
 #pragma unroll
         for (int d = 0; d < DM; ++d) {
-            const double a = A.alpha[d][t], s = a * A.theta, r = 1.0 / a;
+            const double a = in(A.alpha[d], t), s = a * A.theta, r = 1.0 / a;
             put(A.o_alpha[d], A.f_alpha[d], t, s);
             put(A.o_ainv[d], A.f_ainv[d], t, r);
             ds = ds || differs(s, s0);
@@ -61,12 +65,12 @@ __global__ void __launch_bounds__(kT) k_coeffs_fine(CoefFine A) {
             if constexpr (W)
                 if (A.o_pa[d]) put(A.o_pa[d], A.f_pa[d], t, (((A.D.wall >> d) & 1) && x[d] == 0) ? 0.0 : r);
         }
-        put(A.o_beta, A.f_beta, t, A.beta[t]);
-        put(A.o_gamma, A.f_gamma, t, A.gamma ? A.gamma[t] : 0.0);
+        put(A.o_beta, A.f_beta, t, in(A.beta, t));
+        put(A.o_gamma, A.f_gamma, t, A.gamma ? in(A.gamma, t) : 0.0);
     }
 #pragma unroll
     for (int e = 0; e < (DM == 2 ? 1 : 3); ++e)
-        if (t < A.ne[e]) put(A.o_bed[e], A.f_bed[e], t, A.bed[e][t]);
+        if (t < A.ne[e]) put(A.o_bed[e], A.f_bed[e], t, in(A.bed[e], t));
     raise(ds, A.flag_a);
     raise(dr, A.flag_p);
     if (t == 0) {
@@ -78,7 +82,7 @@ __global__ void __launch_bounds__(kT) k_coeffs_fine(CoefFine A) {
 // the mean of the fine faces a coarse face of component d covers
 template <int DM>
 __device__ __forceinline__ double face_mean(const double* a, const Dims& F, int d, int I, int J, int K) {
-    auto at = [&](int i, int j, int k) { return __ldg(a + (i + (int64_t)F.nx * (j + (int64_t)F.ny * k))); };
+    auto at = [&](int i, int j, int k) { return ld(a, i + F.nx * (j + F.ny * k)); };
     if constexpr (DM == 2)
         return d == 0 ? 0.5 * (at(I, J, K) + at(I, J + 1, K)) : 0.5 * (at(I, J, K) + at(I + 1, J, K));
     if (d == 0) return 0.25 * (at(I, J, K) + at(I, J + 1, K) + at(I, J, K + 1) + at(I, J + 1, K + 1));
@@ -87,7 +91,7 @@ __device__ __forceinline__ double face_mean(const double* a, const Dims& F, int 
 }
 template <int DM>
 __device__ __forceinline__ double cell_mean(const double* a, const Dims& F, int I, int J, int K) {
-    auto at = [&](int i, int j, int k) { return __ldg(a + (i + (int64_t)F.nx * (j + (int64_t)F.ny * k))); };
+    auto at = [&](int i, int j, int k) { return ld(a, i + F.nx * (j + F.ny * k)); };
     if constexpr (DM == 2) return 0.25 * (at(I, J, K) + at(I + 1, J, K) + at(I, J + 1, K) + at(I + 1, J + 1, K));
     return 0.125 * (at(I, J, K) + at(I + 1, J, K) + at(I, J + 1, K) + at(I + 1, J + 1, K) + at(I, J, K + 1) + at(I + 1, J, K + 1) +
                     at(I, J + 1, K + 1) + at(I + 1, J + 1, K + 1));
@@ -139,7 +143,7 @@ __global__ void __launch_bounds__(kT) k_coeffs_coarse(CoefCoarse A) {
             const int cx = edge_ext(C, e, 0), cy = edge_ext(C, e, 1), cz = DM == 3 ? edge_ext(C, e, 2) : C.nz;
             if (i >= cx || j >= cy || k >= cz) continue;
             const int fx = edge_ext(F, e, 0), fy = edge_ext(F, e, 1);
-            auto at = [&](int a, int b, int c) { return __ldg(A.bed[e] + (a + (int64_t)fx * (b + (int64_t)fy * c))); };
+            auto at = [&](int a, int b, int c) { return ld(A.bed[e], a + fx * (b + fy * c)); };
             double v;
             if (DM == 2)
                 v = at(I, J, K);

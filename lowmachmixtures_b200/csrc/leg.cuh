@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kLegThreads, 1) k_level_leg(const __grid_const
         const int64_t g = io + at[u];
 #pragma unroll
         for (int d = 0; d < DM; ++d) {
-            const T f0 = A.rhs[d][g], f1 = A.rhs[d][g + 1];
+            const T f0 = ldp<1>(A.rhs[d], (int)g), f1 = ldp<1>(A.rhs[d], (int)g + 1);
             rhs[d * rp + E[u].r] = p ? f1 : f0;
             rhs[d * rp + O[u].r] = p ? f0 : f1;
         }
@@ -230,8 +230,8 @@ __global__ void __launch_bounds__(kLegThreads, 1) k_level_leg(const __grid_const
             T v[3][2] = {};
 #pragma unroll
             for (int d = 0; d < DM; ++d) {
-                v[d][0] = A.phi[d][g];
-                v[d][1] = A.phi[d][g + 1];
+                v[d][0] = ldp<1>(A.phi[d], (int)g);
+                v[d][1] = ldp<1>(A.phi[d], (int)g + 1);
             }
             if (A.up) prolong_cells<T, DM, W>(Dc, A.cphi[0] + ic, A.cphi[1] + ic, A.cphi[DM - 1] + ic, h, j, k, v);
 #pragma unroll

@@ -26,6 +26,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <optional>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -329,6 +330,10 @@ struct lmm_handle {
     const double** gtab_host = nullptr;       // pinned
     double* bslot(int k) { return bslots + (int64_t)k * batch * 8; }
 
+    bool in_arena(const void* p) const {
+        const char* c = static_cast<const char*>(p);
+        return c >= arena && c < arena + arena_bytes;
+    }
     template <class T>
     T* alloc(int64_t count) {
         size_t bytes = ((size_t)count * sizeof(T) + 255) & ~(size_t)255;
@@ -684,6 +689,7 @@ void load_coeffs(lmm_handle* h, const double* const alpha_dev[3], const double* 
     LevelDev<double>& L0 = h->L64[0];
     // an array the kernels cannot read where it is goes to the level's own first
     CallerArrays arrays(h);
+    std::optional<BcScope> faces, edges[3];
     auto at = [&](const double* src, double* own, int64_t count) -> const double* {
         if (src == own || arrays.in_place(src, count * sizeof(double))) return src;
         copy_array(h, own, src, count);
@@ -732,6 +738,13 @@ void load_coeffs(lmm_handle* h, const double* const alpha_dev[3], const double* 
             for (int e = 0; e < nedge; ++e) A.f_bed[e] = f.bed[e];
         }
         slots(0, A.val_a, A.val_p, A.flag_a, A.flag_p);
+        // the caller's arrays, until the wait below
+        auto outside = [&](const double* p) { return h->in_arena(p) ? nullptr : p; };
+        faces.emplace(std::initializer_list<const void*>{outside(A.alpha[0]), outside(A.alpha[1]), outside(A.alpha[2]), outside(A.beta),
+                                                         outside(A.gamma)},
+                      h->n * sizeof(double));
+        for (int e = 0; e < nedge; ++e)
+            edges[e].emplace(std::initializer_list<const void*>{outside(A.bed[e])}, A.ne[e] * sizeof(double));
         launch_coeffs_fine(A, h->stream);
         check_launch();
     }

@@ -34,8 +34,10 @@ namespace lmm {
 // global address must lie in one of the registered device allocations (the
 // arenas and learned-stage blocks of the live handles, and the caller's
 // arrays of an entry point that reads them in place), a shared-memory one
-// (the single-CTA coarse tails) within the CTA's shared memory.  A load outside them is skipped
-// (it reads zero), counted, and the first such address kept; the host reads
+// (the coarse tails, the cluster legs) within the CTA's shared memory; a store
+// into another block's shared memory (dsmem_store) is tested likewise.  An
+// access outside them is skipped (a load reads zero), counted, and the first
+// such address kept; the host reads
 // and clears the record after each solve and reports LMM_ERR_BOUNDS.  Device
 // globals are per translation unit (no relocatable device code), so each
 // unit that includes this header owns a table and a record, reached through
@@ -57,18 +59,29 @@ static __device__ bc::Record g_bc_record;
 // shared memory (static + dynamic), in global memory within a registered
 // allocation; other windows (local) are not tracked.  A call, not inlined: it
 // sits behind every load, and inlined it is most of this build's compile time.
+//
+// A shared-memory address, this block's or another's of its cluster: a block's
+// shared memory (static, then dynamic) follows the reserved region, offsets
+// [cap, cap + total).  In a cluster the window holds every block's, and the
+// offset is the low 24 bits: what addresses of a 16-block cluster looked like
+// on sm_100, not a documented layout.  Another layout would report accesses
+// that are in range; it could not hide one within a block's own memory.
+__device__ __forceinline__ bool bc_in_shared(unsigned a, unsigned bytes) {
+    unsigned total, cap;
+    asm("mov.u32 %0, %%total_smem_size;" : "=r"(total));
+    asm("mov.u32 %0, %%reserved_smem_offset_cap;" : "=r"(cap));
+    const unsigned long long off = a & 0xffffffu;
+    return off >= cap && off + bytes <= (unsigned long long)cap + total;
+}
+__device__ __forceinline__ bool bc_record(bool ok, unsigned long long a) {
+    if (!ok && atomicAdd(&g_bc_record.count, 1ull) == 0ull) g_bc_record.first = a;
+    return ok;
+}
 static __device__ __noinline__ bool bc_ok(const void* p, unsigned bytes) {
     const unsigned long long a = reinterpret_cast<unsigned long long>(p);
     bool ok;
     if (__isShared(p)) {
-        // the CTA's own shared memory (static, then dynamic) follows the
-        // reserved region: offsets [cap, cap + total).  In a cluster the window
-        // holds every CTA's, 16 MB apart: the offset is the low 24 bits
-        unsigned total, cap;
-        asm("mov.u32 %0, %%total_smem_size;" : "=r"(total));
-        asm("mov.u32 %0, %%reserved_smem_offset_cap;" : "=r"(cap));
-        const unsigned long long off = __cvta_generic_to_shared(p) & 0xffffffull;
-        ok = off >= cap && off + bytes <= (unsigned long long)cap + total;
+        ok = bc_in_shared((unsigned)__cvta_generic_to_shared(p), bytes);
     } else if (__isGlobal(p)) {
         ok = false;
         const int n = g_bc_table.n;
@@ -76,9 +89,9 @@ static __device__ __noinline__ bool bc_ok(const void* p, unsigned bytes) {
     } else {
         ok = true;
     }
-    if (!ok && atomicAdd(&g_bc_record.count, 1ull) == 0ull) g_bc_record.first = a;
-    return ok;
+    return bc_record(ok, a);
 }
+static __device__ __noinline__ bool bc_cluster_ok(unsigned a, unsigned bytes) { return bc_record(bc_in_shared(a, bytes), a); }
 #define LMM_BC_UNIT(name)                                                                             \
     cudaError_t lmm_bc_sync_##name(const lmm::bc::Table& t) {                                         \
         return cudaMemcpyToSymbol(lmm::g_bc_table, &t, sizeof(t));                                    \
