@@ -27,6 +27,7 @@ struct LevelDev {
     T* phi[3];
     T* rhs[3];
     T* tmp[3];          // Jacobi output / scratch
+    bool leg;           // leg_supported for the handle's visc_type
     // pressure (cell-centred) multigrid level
     T* pa[3];           // face coefficient 1/alpha (coarsened)
     // every entry of pa holds the same value pa_value (checked on the
@@ -138,7 +139,8 @@ bool launch_residual_pairs(const LevelDev<T>& L, int visc, const T* const rhs[3]
 // One level's leg of a V-cycle in one launch of a thread-block cluster
 // (leg.cuh).  Down: nsm smooths of L (zero: from phi = 0), the residual and
 // its restriction to Cc.rhs; up: the prolongation of Cc.phi and nsm smooths.
-// Gauss-Seidel levels of even sizes whose cells a cluster's threads can own.
+// Gauss-Seidel levels of even sizes whose cells a cluster's threads can own,
+// on a device that can hold such a cluster (a query; LevelDev::leg keeps it).
 template <class T>
 bool leg_supported(const LevelDev<T>& L, int visc);
 template <class T>

@@ -320,35 +320,50 @@ LegShape leg_shape(const LevelDev<T>& L, int visc) {
     return r;
 }
 
+// fits null: the launch; else asks whether the device can hold its cluster
 template <class K, class A>
-static cudaError_t launch_leg_k(K kernel, const A& args, const LegShape& sh, int blocks, cudaStream_t s) {
+static cudaError_t launch_leg_k(K kernel, const A& args, const LegShape& sh, int blocks, cudaStream_t s, bool* fits) {
     cudaError_t e = raise_smem_limit((const void*)kernel, std::max<size_t>(sh.smem, 49152));
     if (e != cudaSuccess) return e;
     if (sh.nc > 8) {
         e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
-    return launch_cluster(kernel, dim3(blocks * sh.nc), dim3(sh.threads), dim3(sh.nc), sh.smem, s, args);
+    const dim3 grid(blocks * sh.nc), block(sh.threads), nc(sh.nc);
+    if (fits) {
+        *fits = cluster_fits(kernel, grid, block, nc, sh.smem);
+        return cudaSuccess;
+    }
+    return launch_cluster(kernel, grid, block, nc, sh.smem, s, args);
 }
 
 template <class T, int DM, bool W, int PP>
-static cudaError_t launch_leg_v(int visc, const LegArgs<T>& a, const LegShape& sh, int blocks, cudaStream_t s) {
+static cudaError_t launch_leg_v(int visc, const LegArgs<T>& a, const LegShape& sh, int blocks, cudaStream_t s, bool* fits) {
     switch (visc) {
-        case -1: return launch_leg_k(k_level_leg<T, DM, -1, W, PP>, a, sh, blocks, s);
-        case -2: return launch_leg_k(k_level_leg<T, DM, -2, W, PP>, a, sh, blocks, s);
-        default: return launch_leg_k(k_level_leg<T, DM, -3, W, PP>, a, sh, blocks, s);
+        case -1: return launch_leg_k(k_level_leg<T, DM, -1, W, PP>, a, sh, blocks, s, fits);
+        case -2: return launch_leg_k(k_level_leg<T, DM, -2, W, PP>, a, sh, blocks, s, fits);
+        default: return launch_leg_k(k_level_leg<T, DM, -3, W, PP>, a, sh, blocks, s, fits);
     }
 }
 template <class T, int DM, bool W>
-static cudaError_t launch_leg_p(int visc, const LegArgs<T>& a, const LegShape& sh, int blocks, cudaStream_t s) {
+static cudaError_t launch_leg_p(int visc, const LegArgs<T>& a, const LegShape& sh, int blocks, cudaStream_t s, bool* fits) {
     if constexpr (sizeof(T) == 4)
-        if (sh.pp == 2) return launch_leg_v<T, DM, W, 2>(visc, a, sh, blocks, s);
-    return launch_leg_v<T, DM, W, 1>(visc, a, sh, blocks, s);
+        if (sh.pp == 2) return launch_leg_v<T, DM, W, 2>(visc, a, sh, blocks, s, fits);
+    return launch_leg_v<T, DM, W, 1>(visc, a, sh, blocks, s, fits);
+}
+template <class T>
+static cudaError_t launch_leg(const LevelDev<T>& L, int visc, const LegArgs<T>& a, const LegShape& sh, cudaStream_t s, bool* fits) {
+    const int blocks = L.D.dm == 2 ? L.D.nz : 1;
+    if (L.D.dm == 2)
+        return L.D.wall ? launch_leg_p<T, 2, true>(visc, a, sh, blocks, s, fits) : launch_leg_p<T, 2, false>(visc, a, sh, blocks, s, fits);
+    return L.D.wall ? launch_leg_p<T, 3, true>(visc, a, sh, blocks, s, fits) : launch_leg_p<T, 3, false>(visc, a, sh, blocks, s, fits);
 }
 
 template <class T>
 bool leg_supported(const LevelDev<T>& L, int visc) {
-    return leg_shape<T>(L, visc).nc > 0;
+    const LegShape sh = leg_shape<T>(L, visc);
+    bool fits = false;
+    return sh.nc > 0 && launch_leg<T>(L, visc, LegArgs<T>{}, sh, nullptr, &fits) == cudaSuccess && fits;
 }
 
 template <class T>
@@ -374,10 +389,7 @@ cudaError_t launch_level_leg(const LevelDev<T>& L, const LevelDev<T>& Cc, int vi
         a.cphi[d] = Cc.phi[d];
         a.crhs[d] = Cc.rhs[d];
     }
-    const int blocks = L.D.dm == 2 ? L.D.nz : 1;
-    if (L.D.dm == 2)
-        return L.D.wall ? launch_leg_p<T, 2, true>(visc, a, sh, blocks, s) : launch_leg_p<T, 2, false>(visc, a, sh, blocks, s);
-    return L.D.wall ? launch_leg_p<T, 3, true>(visc, a, sh, blocks, s) : launch_leg_p<T, 3, false>(visc, a, sh, blocks, s);
+    return launch_leg<T>(L, visc, a, sh, s, nullptr);
 }
 
 #define LMM_INSTANTIATE_LEG(T)                                                  \

@@ -505,6 +505,7 @@ void build_levels(lmm_handle* h) {
                 v.tmp[d] = h->alloc<T>(v.n);
             }
         }
+        v.leg = !h->batched && l + 1 < h->nlev && leg_supported<T>(v, h->knobs.visc_type);
         if (l < h->nlev_p) {
             // the finest level of a periodic box shares 1/alpha (create_impl)
             if (l > 0 || h->D0.wall)
@@ -1038,7 +1039,7 @@ template <class T>
 bool use_leg(const lmm_handle* h, const LevelDev<T>& L) {
     const lmm_knobs& K = h->knobs;
     return K.tail_cells >= 0 && K.stag_mg_smoother != 0 && K.smoother_fusion <= 0 && K.residual_fusion <= 0 && !h->batched &&
-           !use_tma_smoother<T>(h, L) && leg_supported<T>(L, K.visc_type);
+           !use_tma_smoother<T>(h, L) && L.leg;
 }
 
 // one V-cycle on L[0].phi / L[0].rhs; zero: from L[0].phi = 0, whatever the
