@@ -47,42 +47,24 @@ __device__ __forceinline__ void dsmem_store(unsigned a, double v) {
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
-// a launch of clusters of nc.x x nc.y x nc.z blocks, ranked x fastest (each extent of the grid a multiple of its)
-struct ClusterConfig {
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at[2];
-    ClusterConfig(dim3 grid, dim3 block, dim3 nc, size_t smem, cudaStream_t s) {
-        cfg.gridDim = grid;
-        cfg.blockDim = block;
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[0].val.programmaticStreamSerializationAllowed = 1;
-        at[1].id = cudaLaunchAttributeClusterDimension;
-        at[1].val.clusterDim.x = nc.x;
-        at[1].val.clusterDim.y = nc.y;
-        at[1].val.clusterDim.z = nc.z;
-        cfg.attrs = at;
-        cfg.numAttrs = 2;
-    }
-    ClusterConfig(const ClusterConfig&) = delete;
-    ClusterConfig& operator=(const ClusterConfig&) = delete;
-};
+// clusters of nc.x x nc.y x nc.z blocks, ranked x fastest (each extent of the grid a multiple of its)
 template <class... KArgs, class... Args>
 static inline cudaError_t launch_cluster(void (*k)(KArgs...), dim3 grid, dim3 block, dim3 nc, size_t smem, cudaStream_t s, Args... args) {
-    const ClusterConfig c(grid, block, nc, smem, s);
-    return cudaLaunchKernelEx(&c.cfg, k, args...);
-}
-// the device (or the part of it that this process has) can hold such a cluster
-template <class... KArgs>
-static inline bool cluster_fits(void (*k)(KArgs...), dim3 grid, dim3 block, dim3 nc, size_t smem) {
-    const ClusterConfig c(grid, block, nc, smem, nullptr);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k, &c.cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return n > 0;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = nc.x;
+    at[1].val.clusterDim.y = nc.y;
+    at[1].val.clusterDim.z = nc.z;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
 }  // namespace lmm

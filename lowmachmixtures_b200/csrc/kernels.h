@@ -27,7 +27,7 @@ struct LevelDev {
     T* phi[3];
     T* rhs[3];
     T* tmp[3];          // Jacobi output / scratch
-    bool leg;           // leg_supported for the handle's visc_type
+    int leg;            // leg_supported for the handle's visc_type: 1 yes, -1 no, 0 not asked yet
     // pressure (cell-centred) multigrid level
     T* pa[3];           // face coefficient 1/alpha (coarsened)
     // every entry of pa holds the same value pa_value (checked on the
@@ -140,7 +140,7 @@ bool launch_residual_pairs(const LevelDev<T>& L, int visc, const T* const rhs[3]
 // (leg.cuh).  Down: nsm smooths of L (zero: from phi = 0), the residual and
 // its restriction to Cc.rhs; up: the prolongation of Cc.phi and nsm smooths.
 // Gauss-Seidel levels of even sizes whose cells a cluster's threads can own,
-// on a device that can hold such a cluster (a query; LevelDev::leg keeps it).
+// on a device that can hold such a cluster (LevelDev::leg keeps the answer).
 template <class T>
 bool leg_supported(const LevelDev<T>& L, int visc);
 template <class T>
@@ -208,6 +208,9 @@ int reduce_blocks(int64_t n);
 // raise a kernel's dynamic shared-memory limit to at least `bytes` on the
 // current device, once per (device, kernel); safe from several host threads
 cudaError_t raise_smem_limit(const void* kernel, size_t bytes);
+// the current device (or the part of it that this process has) can hold one
+// cluster of nc blocks of this kernel; asked once per (device, kernel, shape)
+bool cluster_fits(const void* kernel, int nc, int threads, size_t smem);
 
 // bounds-check builds (-DLMM_BOUNDS_CHECK, stencil.cuh): register / forget a
 // device allocation that loads may touch; bc_status reads and clears every

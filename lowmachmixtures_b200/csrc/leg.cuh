@@ -331,7 +331,7 @@ static cudaError_t launch_leg_k(K kernel, const A& args, const LegShape& sh, int
     }
     const dim3 grid(blocks * sh.nc), block(sh.threads), nc(sh.nc);
     if (fits) {
-        *fits = cluster_fits(kernel, grid, block, nc, sh.smem);
+        *fits = cluster_fits((const void*)kernel, sh.nc, sh.threads, sh.smem);
         return cudaSuccess;
     }
     return launch_cluster(kernel, grid, block, nc, sh.smem, s, args);

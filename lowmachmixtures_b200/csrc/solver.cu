@@ -505,7 +505,6 @@ void build_levels(lmm_handle* h) {
                 v.tmp[d] = h->alloc<T>(v.n);
             }
         }
-        v.leg = !h->batched && l + 1 < h->nlev && leg_supported<T>(v, h->knobs.visc_type);
         if (l < h->nlev_p) {
             // the finest level of a periodic box shares 1/alpha (create_impl)
             if (l > 0 || h->D0.wall)
@@ -1034,12 +1033,16 @@ int tail_start(lmm_handle* h, const std::vector<LevelDev<T>>& L, int nl, bool st
     return lc;
 }
 
-// the level's legs of a V-cycle run as cluster launches (leg.cuh)
+// the level's legs of a V-cycle run as cluster launches (leg.cuh).  What the
+// device can hold is asked by the handle's first V-cycle, which is never captured.
 template <class T>
-bool use_leg(const lmm_handle* h, const LevelDev<T>& L) {
+bool use_leg(const lmm_handle* h, LevelDev<T>& L) {
     const lmm_knobs& K = h->knobs;
-    return K.tail_cells >= 0 && K.stag_mg_smoother != 0 && K.smoother_fusion <= 0 && K.residual_fusion <= 0 && !h->batched &&
-           !use_tma_smoother<T>(h, L) && L.leg;
+    if (K.tail_cells < 0 || K.stag_mg_smoother == 0 || K.smoother_fusion > 0 || K.residual_fusion > 0 || h->batched ||
+        use_tma_smoother<T>(h, L))
+        return false;
+    if (L.leg == 0) L.leg = leg_supported<T>(L, K.visc_type) ? 1 : -1;
+    return L.leg > 0;
 }
 
 // one V-cycle on L[0].phi / L[0].rhs; zero: from L[0].phi = 0, whatever the
@@ -3379,6 +3382,32 @@ cudaError_t raise_smem_limit(const void* kernel, size_t bytes) {
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e == cudaSuccess) cur = bytes;
     return e;
+}
+bool cluster_fits(const void* kernel, int nc, int threads, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, const void*, int, int, size_t>, bool> known;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_tuple(dev, kernel, nc, threads, smem);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = nc;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nc);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    return known[key] = n > 0;
 }
 int64_t launches_total() { return g_launches.load(std::memory_order_relaxed); }
 int reduce_blocks(int64_t n) {
