@@ -102,8 +102,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 5 : 0) k_applyop(Di
 }
 
 // --------------------------------------------------------------- one component per thread
-// The same face values as k_applyop (colour 0) and k_residual with one face
-// component per thread: grid.z covers nz * DM, component = blockIdx.z % DM
+// The face values of k_applyop (colour 0), and the residual r = (L phi - rhs) * -1
+// (stag_mg_solver.f90:406-415; W: zero on wall faces, physbc_domainvel,
+// stag_mg_solver.f90:424-425), with one face component per thread: grid.z covers nz * DM, component = blockIdx.z % DM
 // (uniform per block), so a thread keeps one stencil live instead of DM.
 struct PosC {
     int i, j, k, comp;
@@ -381,42 +382,6 @@ __device__ __forceinline__ T fine_resid(const Dims& F, const Coef<T>& C, const T
     Nb nb = make_nb(F, i, j, k);
     T v = face_L<T, DM, VISC, D_, LD>(phi, C, nb, dxsqinv, b, c) - ldp<LD>(rhs, nb.s);
     return v * T(-1);
-}
-
-// r = (L phi - rhs) * -1 on every face of one level (stag_mg_solver.f90:406-415)
-// W: the residual is zero on wall faces (physbc_domainvel, stag_mg_solver.f90:424-425)
-template <class T, int DM, int VISC, bool W = false>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 5 : 0) k_residual(Dims D, Coef<T> C, const T* __restrict__ r0, const T* __restrict__ r1,
-                                                       const T* __restrict__ r2, const T* __restrict__ p0, const T* __restrict__ p1,
-                                                       const T* __restrict__ p2, T* __restrict__ o0, T* __restrict__ o1,
-                                                       T* __restrict__ o2, T dxsqinv) {
-    pdl_enter();
-    const Pos q = pos3(D.nx, D.ny);
-    if (!q.ok) return;
-    Nb nb = W ? make_nbw(D, q.i, q.j, q.k) : make_nb(D, q.i, q.j, q.k);
-    const int t = nb.s;
-    const T* phi[3] = {p0, p1, p2};
-    const T b = ld(C.beta, 0), c = ld(C.gamma, 0);
-    if (W && wall_face(nb, 0)) {
-        o0[t] = T(0);
-    } else {
-        T v = face_L<T, DM, VISC, 0, 0, T, W>(phi, C, nb, dxsqinv, b, c) - ld(r0, t);
-        o0[t] = v * T(-1);
-    }
-    if (W && wall_face(nb, 1)) {
-        o1[t] = T(0);
-    } else {
-        T v = face_L<T, DM, VISC, 1, 0, T, W>(phi, C, nb, dxsqinv, b, c) - ld(r1, t);
-        o1[t] = v * T(-1);
-    }
-    if constexpr (DM == 3) {
-        if (W && wall_face(nb, 2)) {
-            o2[t] = T(0);
-        } else {
-            T v = face_L<T, DM, VISC, 2, 0, T, W>(phi, C, nb, dxsqinv, b, c) - ld(r2, t);
-            o2[t] = v * T(-1);
-        }
-    }
 }
 
 // 6-point (2D) / 12-point (3D) restriction of precomputed fine residuals of

@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kLegThreads, 1) k_level_leg(const __grid_const
     extern __shared__ __align__(16) unsigned char leg_smem[];
     T* sm = reinterpret_cast<T*>(leg_smem);
     constexpr int SD = DM - 1;
-    const int NC = A.nc, rank = (int)cluster_rank(), inst = DM == 2 ? (int)blockIdx.x / NC : 0;
+    const int NC = A.nc, rank = (int)cluster_rank();
     const int plane = DM == 3 ? A.D.nx * A.D.ny : A.D.nx, S = DM == 3 ? A.D.nz : A.D.ny;
     const int half = A.D.nx >> 1, hplane = plane >> 1;
     const int z0 = rank * S / NC, z1 = (rank + 1) * S / NC, t = z1 - z0;
@@ -152,19 +152,7 @@ __global__ void __launch_bounds__(kLegThreads, 1) k_level_leg(const __grid_const
     L.D = A.D;
     L.dxsqinv = A.dxsqinv;
     L.C = A.C;
-    Dims Dc = A.Dc;
-    int64_t io = 0, ic = 0;
-    if constexpr (DM == 2) {
-        io = (int64_t)inst * A.D.nx * A.D.ny;
-        ic = (int64_t)inst * A.Dc.nx * A.Dc.ny;
-        const int64_t ie = (int64_t)inst * edge_ext(A.D, 0, 0) * edge_ext(A.D, 0, 1);
-        L.D.nz = Dc.nz = 1;
-        L.C.alpha[0] = shift(A.C.alpha[0], io);
-        L.C.alpha[1] = shift(A.C.alpha[1], io);
-        L.C.bed[0] = shift(A.C.bed[0], ie);
-        L.C.beta = shift(A.C.beta, io);
-        L.C.gamma = shift(A.C.gamma, io);
-    }
+    const Dims Dc = A.Dc;
     // the coefficients, ahead of the wait for the previous kernel: they are
     // written once per coefficient load, never by the launch before this one
     const T b = ld(L.C.beta, 0), c = ld(L.C.gamma, 0);
@@ -219,10 +207,10 @@ __global__ void __launch_bounds__(kLegThreads, 1) k_level_leg(const __grid_const
     for (int u = 0; u < PP; ++u) {
         if (!E[u].o.on) continue;
         const int j = jk[u] & 0xffff, k = jk[u] >> 16, p = (j + k) & 1, h = (at[u] % A.D.nx) >> 1;
-        const int64_t g = io + at[u];
+        const int g = at[u];
 #pragma unroll
         for (int d = 0; d < DM; ++d) {
-            const T f0 = ldp<1>(A.rhs[d], (int)g), f1 = ldp<1>(A.rhs[d], (int)g + 1);
+            const T f0 = ldp<1>(A.rhs[d], g), f1 = ldp<1>(A.rhs[d], g + 1);
             rhs[d * rp + E[u].r] = p ? f1 : f0;
             rhs[d * rp + O[u].r] = p ? f0 : f1;
         }
@@ -230,10 +218,10 @@ __global__ void __launch_bounds__(kLegThreads, 1) k_level_leg(const __grid_const
             T v[3][2] = {};
 #pragma unroll
             for (int d = 0; d < DM; ++d) {
-                v[d][0] = ldp<1>(A.phi[d], (int)g);
-                v[d][1] = ldp<1>(A.phi[d], (int)g + 1);
+                v[d][0] = ldp<1>(A.phi[d], g);
+                v[d][1] = ldp<1>(A.phi[d], g + 1);
             }
-            if (A.up) prolong_cells<T, DM, W>(Dc, A.cphi[0] + ic, A.cphi[1] + ic, A.cphi[DM - 1] + ic, h, j, k, v);
+            if (A.up) prolong_cells<T, DM, W>(Dc, A.cphi[0], A.cphi[1], A.cphi[DM - 1], h, j, k, v);
 #pragma unroll
             for (int d = 0; d < DM; ++d) {
                 E[u].put(sm, pitch, hp, d, p ? v[d][1] : v[d][0]);
@@ -260,7 +248,7 @@ __global__ void __launch_bounds__(kLegThreads, 1) k_level_leg(const __grid_const
     for (int u = 0; u < PP; ++u) {
         if (!E[u].o.on) continue;
         const int p = ((jk[u] & 0xffff) + (jk[u] >> 16)) & 1;
-        const int64_t g = io + at[u];
+        const int g = at[u];
 #pragma unroll
         for (int d = 0; d < DM; ++d) {
             A.phi[d][g + p] = sm[d * pitch + E[u].o.s];
@@ -284,11 +272,11 @@ __global__ void __launch_bounds__(kLegThreads, 1) k_level_leg(const __grid_const
         int i, j, k;
         unflat3d(Dc, w, i, j, k);
         if (comp == 0)
-            A.crhs[0][ic + w] = restrict_one<T, DM, 0, W, 2>(L.D, A.tmp[0] + io, Dc, i, j, k);
+            A.crhs[0][w] = restrict_one<T, DM, 0, W, 2>(L.D, A.tmp[0], Dc, i, j, k);
         else if (comp == 1)
-            A.crhs[1][ic + w] = restrict_one<T, DM, 1, W, 2>(L.D, A.tmp[1] + io, Dc, i, j, k);
+            A.crhs[1][w] = restrict_one<T, DM, 1, W, 2>(L.D, A.tmp[1], Dc, i, j, k);
         else if constexpr (DM == 3)
-            A.crhs[2][ic + w] = restrict_one<T, DM, 2, W, 2>(L.D, A.tmp[2] + io, Dc, i, j, k);
+            A.crhs[2][w] = restrict_one<T, DM, 2, W, 2>(L.D, A.tmp[2], Dc, i, j, k);
     }
 }
 
@@ -300,7 +288,7 @@ struct LegShape {
 template <class T>
 LegShape leg_shape(const LevelDev<T>& L, int visc) {
     LegShape r;
-    if (visc >= 0 || odd_level(L.D)) return r;
+    if (visc >= 0 || odd_level(L.D) || (L.D.dm == 2 && L.D.nz != 1)) return r;   // (a batch stacks nz instances)
     const int dm = L.D.dm, plane = dm == 3 ? L.D.nx * L.D.ny : L.D.nx, S = dm == 3 ? L.D.nz : L.D.ny;
     for (int nc : {8, 16}) {
         const int t = (S + nc - 1) / nc;
@@ -322,41 +310,40 @@ LegShape leg_shape(const LevelDev<T>& L, int visc) {
 
 // fits null: the launch; else asks whether the device can hold its cluster
 template <class K, class A>
-static cudaError_t launch_leg_k(K kernel, const A& args, const LegShape& sh, int blocks, cudaStream_t s, bool* fits) {
+static cudaError_t launch_leg_k(K kernel, const A& args, const LegShape& sh, cudaStream_t s, bool* fits) {
     cudaError_t e = raise_smem_limit((const void*)kernel, std::max<size_t>(sh.smem, 49152));
     if (e != cudaSuccess) return e;
     if (sh.nc > 8) {
         e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
-    const dim3 grid(blocks * sh.nc), block(sh.threads), nc(sh.nc);
+    const dim3 nc(sh.nc), block(sh.threads);   // one cluster
     if (fits) {
         *fits = cluster_fits((const void*)kernel, sh.nc, sh.threads, sh.smem);
         return cudaSuccess;
     }
-    return launch_cluster(kernel, grid, block, nc, sh.smem, s, args);
+    return launch_cluster(kernel, nc, block, nc, sh.smem, s, args);
 }
 
 template <class T, int DM, bool W, int PP>
-static cudaError_t launch_leg_v(int visc, const LegArgs<T>& a, const LegShape& sh, int blocks, cudaStream_t s, bool* fits) {
+static cudaError_t launch_leg_v(int visc, const LegArgs<T>& a, const LegShape& sh, cudaStream_t s, bool* fits) {
     switch (visc) {
-        case -1: return launch_leg_k(k_level_leg<T, DM, -1, W, PP>, a, sh, blocks, s, fits);
-        case -2: return launch_leg_k(k_level_leg<T, DM, -2, W, PP>, a, sh, blocks, s, fits);
-        default: return launch_leg_k(k_level_leg<T, DM, -3, W, PP>, a, sh, blocks, s, fits);
+        case -1: return launch_leg_k(k_level_leg<T, DM, -1, W, PP>, a, sh, s, fits);
+        case -2: return launch_leg_k(k_level_leg<T, DM, -2, W, PP>, a, sh, s, fits);
+        default: return launch_leg_k(k_level_leg<T, DM, -3, W, PP>, a, sh, s, fits);
     }
 }
 template <class T, int DM, bool W>
-static cudaError_t launch_leg_p(int visc, const LegArgs<T>& a, const LegShape& sh, int blocks, cudaStream_t s, bool* fits) {
+static cudaError_t launch_leg_p(int visc, const LegArgs<T>& a, const LegShape& sh, cudaStream_t s, bool* fits) {
     if constexpr (sizeof(T) == 4)
-        if (sh.pp == 2) return launch_leg_v<T, DM, W, 2>(visc, a, sh, blocks, s, fits);
-    return launch_leg_v<T, DM, W, 1>(visc, a, sh, blocks, s, fits);
+        if (sh.pp == 2) return launch_leg_v<T, DM, W, 2>(visc, a, sh, s, fits);
+    return launch_leg_v<T, DM, W, 1>(visc, a, sh, s, fits);
 }
 template <class T>
 static cudaError_t launch_leg(const LevelDev<T>& L, int visc, const LegArgs<T>& a, const LegShape& sh, cudaStream_t s, bool* fits) {
-    const int blocks = L.D.dm == 2 ? L.D.nz : 1;
     if (L.D.dm == 2)
-        return L.D.wall ? launch_leg_p<T, 2, true>(visc, a, sh, blocks, s, fits) : launch_leg_p<T, 2, false>(visc, a, sh, blocks, s, fits);
-    return L.D.wall ? launch_leg_p<T, 3, true>(visc, a, sh, blocks, s, fits) : launch_leg_p<T, 3, false>(visc, a, sh, blocks, s, fits);
+        return L.D.wall ? launch_leg_p<T, 2, true>(visc, a, sh, s, fits) : launch_leg_p<T, 2, false>(visc, a, sh, s, fits);
+    return L.D.wall ? launch_leg_p<T, 3, true>(visc, a, sh, s, fits) : launch_leg_p<T, 3, false>(visc, a, sh, s, fits);
 }
 
 template <class T>

@@ -1,11 +1,17 @@
 // pdl.cuh - programmatic dependent launch.
 //
-// A kernel launched with launch_pdl may be scheduled while the kernel before
-// it on the stream drains; its first statement, pdl_enter(), waits for that
-// kernel's completion and memory (griddepcontrol.wait) before any access,
-// then lets the next kernel be scheduled (griddepcontrol.launch_dependents).
-// Launched without the attribute, both instructions are no-ops.  Every
-// kernel launched through launch_pdl starts with pdl_enter().
+// A kernel launched with launch_pdl (or launch_cluster) may be scheduled while
+// the kernel before it on the stream drains; pdl_enter() waits for that
+// kernel's completion and memory (griddepcontrol.wait), then lets the next
+// kernel be scheduled (griddepcontrol.launch_dependents).  Launched without the
+// attribute, both instructions are no-ops.  Every kernel launched so calls it.
+//
+// Since a kernel releases the next one only after its own wait, whatever runs
+// two launches back is complete: before pdl_enter() a kernel may write its own
+// shared memory and read what the launch directly before it does not write,
+// and nothing else.  k_gs_zero, k_cc_zero, k_vcycle_tail, k_ccmg_tail and
+// k_level_leg read coefficients there: these are written by the coefficient
+// load alone, which the host waits for before it launches any of them.
 #pragma once
 #include <cuda_runtime.h>
 
