@@ -857,16 +857,6 @@ template <int DM, int J, bool NORM>
 int cgs_blocks(int64_t n);
 // blocks of the cluster variant (the grid of one instance is one cluster), 0: too many
 int cgs_cluster(int64_t n) { return mdot_blocks(n) <= 8 ? mdot_blocks(n) : 0; }
-// the grid is split by component too (k_reduce): in one cluster where that still
-// has a portable size, else while the split grid is one wave of three blocks on
-// each of 148 SMs.  A restart cycle's passes: 57.5 us against 75.8 at 2D 256^2 (32
-// blocks), 82.7 / 84.9 at 540 x 560 (148 x 3), 110 / 113 at 60^3 (106 x 4); past it
-// the blocks left over make a second wave: 120 / 113 at 64 x 64 x 56 (112 x 4),
-// 112 / 100 at 64^3
-bool cgs_split(int64_t n, int nc, int ninst) {
-    const int b = mdot_blocks(n);
-    return cgs_cluster(n) ? b * nc <= 8 : (int64_t)b * nc * ninst <= 3 * 148;
-}
 // the Gram-Schmidt passes may take entries in pairs: rows of even length
 // (no pair straddles a row or an instance) and 16-byte aligned vectors
 int pairs_ok(const Dims& D, const void* w, const MVecs& V, int J) {
@@ -881,7 +871,7 @@ void launch_maxpy_norm(const Dims& D, double* w, const MVecs& V, int J, const do
     const int64_t n = (int64_t)D.nx * D.ny * (D.dm == 3 ? D.nz : 1);
     const int vec = pairs_ok(D, w, V, J);
     const int cl = cgs_cluster(n), nc = D.dm + 1;
-    const bool cs = cgs_split(n, nc, ninst);
+    const bool cs = cl ? cl * nc <= 8 : mdot_blocks(n) * ninst <= 148;   // split by component (k_reduce)
 #define MN(DM_, J_)                                                                                                     \
     if (cl && cs)                                                                                                       \
         launch_cluster(k_maxpy_norm<DM_, J_, true, true>, dim3(cl, ninst, nc), dim3(kMdotThreads), dim3(cl, 1, nc), 0, s, D, w, V, hs, wseam, pw, partials, counter, out, ss, vec); \
@@ -939,7 +929,7 @@ void launch_mdot(const Dims& D, const double* w, const MVecs& V, int J, double w
     const int64_t n = (int64_t)D.nx * D.ny * (D.dm == 3 ? D.nz : 1);
     const int vec = pairs_ok(D, w, V, J);
     const int cl = cgs_cluster(n), nc = D.dm + 1;
-    const bool cs = cgs_split(n, nc, ninst);
+    const bool cs = cl ? cl * nc <= 8 : mdot_blocks(n) * ninst <= 148;   // split by component (k_reduce)
 #define MD(DM_, J_)                                                                                                     \
     if (cl && cs)                                                                                                       \
         launch_cluster(k_mdot<DM_, J_, true, true>, dim3(cl, ninst, nc), dim3(kMdotThreads), dim3(cl, 1, nc), 0, s, D, w, V, wseam, pw, partials, counter, out, ss, vec); \

@@ -72,11 +72,10 @@ def test_pairs_equal_single_faces(dm, n, bc, visc):
         np.testing.assert_array_equal(a, b)
 
 
-# blocks of 2048 entries: 1, 2 | 3, 8 (too many to split by component too) | 9 | 111 | 112 (the last split and the
-# first unsplit Gram-Schmidt passes in 3D) | 148 | 149 (likewise the inner products) | 592 (the most); 2D: 147 | 149;
+# blocks of 2048 entries: 1, 2 | 3, 8 (too many to split by component too) | 9 | 148 | 149 | 592 (the most);
 # odd counts read entry by entry
-SIZES = [(2, (16, 16)), (2, (64, 64)), (2, (64, 96)), (2, (128, 128)), (2, (128, 144)), (2, (99, 187)), (2, (540, 556)), (2, (544, 560)),
-         (3, (8, 8, 8)), (3, (16, 16, 16)), (3, (17, 15, 19)), (3, (32, 32, 16)), (3, (32, 24, 24)), (3, (64, 32, 111)), (3, (64, 64, 56)), (3, (64, 64, 74)), (3, (64, 32, 149)),
+SIZES = [(2, (16, 16)), (2, (64, 64)), (2, (64, 96)), (2, (128, 128)), (2, (128, 144)), (2, (99, 187)),
+         (3, (8, 8, 8)), (3, (16, 16, 16)), (3, (17, 15, 19)), (3, (32, 32, 16)), (3, (32, 24, 24)), (3, (64, 64, 74)), (3, (64, 32, 149)),
          (3, (128, 96, 100))]
 
 
