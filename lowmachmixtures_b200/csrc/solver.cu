@@ -426,7 +426,8 @@ size_t plan_bytes(const lmm_grid& g, const lmm_knobs& k, int nlev, int nlev_p, i
                 for (int e = 0; e < ne; ++e) add(edge_count(Dl, e), sz);  // bed (n+1 nodes along walls)
             }
             if (l < nlev_p) {
-                for (int q = 0; q < dm + 3; ++q) add(c, sz);
+                // pa (the finest level of a periodic box shares 1/alpha), pphi, prhs, ptmp
+                for (int q = 0; q < (l > 0 || Dl.wall ? dm : 0) + 3; ++q) add(c, sz);
                 if (k.visc_schur_approx == 1)
                     for (int q = 0; q < dm; ++q) add(c, sz);  // pmu
             }
