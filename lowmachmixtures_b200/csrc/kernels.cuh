@@ -1468,7 +1468,7 @@ void launch_reduce(const Dims& D, int mode, const T* const a[4], const T* const 
     const void* pa[4] = {a[0], a[1], a[2], a[3]};
     const void* pb[4] = {b[0], b[1], b[2], b[3]};
     const int vec = reduce_pairs(D, sizeof(T), pa, pb);
-    // split by component while the grid is smaller than the chip; one cluster (portable size) where the blocks fit
+    // split by component while the grid has no more blocks than the chip SMs (148); one cluster (portable size) where the blocks fit
     const int nc = D.dm + 1, cl = nblocks <= 8 ? nblocks : 0;
     const bool cs = cl ? cl * nc <= 8 : nblocks * ninst <= 148;
 #define RED_ARGS s, D, a[0], a[1], a[2], a[3], b[0], b[1], b[2], b[3], wseam[0], wseam[1], wseam[2], pw, partials, counter, out, vec
